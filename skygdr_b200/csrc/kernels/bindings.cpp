@@ -45,6 +45,15 @@ static LaunchStatus* status_ptr(torch::Tensor& t) {
 }
 
 // A fresh status block: OK, cursor and t_start at their "unset" value of all ones.
+static torch::Tensor new_flow_work(int64_t device) {
+    FlowWork h;
+    memset(&h, 0, sizeof h);
+    h.status.cursor = ~0ull;
+    h.status.t_start_ns = ~0ull;
+    auto cpu = torch::empty({(int64_t)sizeof(FlowWork)}, torch::kUInt8);
+    memcpy(cpu.data_ptr(), &h, sizeof h);
+    return cpu.to(torch::Device(torch::kCUDA, device));
+}
 static torch::Tensor new_status(int64_t device) {
     LaunchStatus h;
     memset(&h, 0, sizeof h);
@@ -61,15 +70,29 @@ static void reset_status(torch::Tensor& t) {
     h.t_start_ns = ~0ull;
     SKY_CUDA_CHECK(cudaMemcpyAsync(t.data_ptr(), &h, sizeof h, cudaMemcpyHostToDevice, cur_stream()));
 }
-static py::dict read_status(const torch::Tensor& t) {
-    auto cpu = t.cpu();
-    LaunchStatus h;
-    memcpy(&h, cpu.data_ptr(), sizeof h);
+static py::dict status_dict(const LaunchStatus& h) {
     py::dict d;
     d["status"] = h.status; d["detail"] = h.detail; d["cursor"] = h.cursor; d["chunks_done"] = h.chunks_done;
     d["bytes_done"] = h.bytes_done; d["stall_ns"] = h.stall_ns; d["t_start_ns"] = h.t_start_ns; d["t_end_ns"] = h.t_end_ns;
     d["ctas_done"] = h.ctas_done;
     return d;
+}
+static py::dict read_status(const torch::Tensor& t) {
+    auto cpu = t.cpu();
+    LaunchStatus h;
+    memcpy(&h, cpu.data_ptr(), sizeof h);
+    return status_dict(h);
+}
+// Waits for the device, then reads the copy of a launch's outcome that its last CTA left in mapped host memory.
+static py::dict sync_and_read_mirror(int64_t device, uint64_t mirror_host_ptr) {
+    {
+        py::gil_scoped_release nogil;
+        c10::cuda::CUDAGuard g((c10::DeviceIndex)device);
+        SKY_CUDA_CHECK(cudaDeviceSynchronize());
+    }
+    LaunchStatus h;
+    memcpy(&h, (const void*)mirror_host_ptr, sizeof h);
+    return status_dict(h);
 }
 
 // ---- mapped host memory (credit pages, offload targets) ----
@@ -187,8 +210,10 @@ static void kv_transfer(torch::Tensor src_pool, std::vector<uint64_t> dst_ptrs, 
                         int block_tokens, int head_dim, std::vector<int64_t> src_strides, std::vector<int64_t> dst_strides,
                         int heads_per_dst, bool replicate, bool fp8, bool keep_layout, int pages_per_chunk, int ctas, uint64_t credit_dev_ptr,
                         uint64_t consumed_base, uint64_t max_wait_ns, uint64_t first_chunk, uint32_t done_value, torch::Tensor status,
-                        bool use_tma, uint64_t multicast_ptr, int src_num_blocks, int dst_num_blocks) {
-    TORCH_CHECK(!(multicast_ptr && (use_tma || fp8 || !replicate)), "a multicast destination takes replicated bf16 pages from the register path");
+                        int use_tma, torch::Tensor work, uint64_t mirror_dev_ptr, int ctas_simt, uint64_t multicast_ptr, int src_num_blocks,
+                        int dst_num_blocks) {
+    // use_tma: 0 the register engine, 1 the copy-hardware engines, 2 those where they take the layout and the register engine elsewhere
+    TORCH_CHECK(!(multicast_ptr && (use_tma == 1 || fp8 || !replicate)), "a multicast destination takes replicated bf16 pages from the register path");
     TORCH_CHECK(dst_ptrs.size() >= 1 && dst_ptrs.size() <= (size_t)KV_MAX_DST, "1..8 destinations");
     TORCH_CHECK(src_strides.size() == 3 && dst_strides.size() == 3, "strides are (block, layer, kv)");
     TORCH_CHECK(src_blocks.numel() == dst_blocks.numel(), "block lists differ in length");
@@ -216,10 +241,15 @@ static void kv_transfer(torch::Tensor src_pool, std::vector<uint64_t> dst_ptrs, 
     p.page = (const SkyCreditPage*)credit_dev_ptr;
     p.usage = (SkyCreditPage*)credit_dev_ptr;
     p.consumed_base = consumed_base; p.max_wait_ns = max_wait_ns; p.first_chunk = first_chunk;
-    p.status = status_ptr(status);
+    TORCH_CHECK(work.is_cuda() && work.is_contiguous() && work.numel() * work.element_size() >= (int64_t)sizeof(FlowWork) && mirror_dev_ptr,
+                "work: a block from new_flow_work; mirror: mapped host memory");
+    FlowWork* fw = reinterpret_cast<FlowWork*>(work.data_ptr());
+    p.status = &fw->status; p.grant = &fw->grant;
+    p.result = status_ptr(status);
+    p.mirror = (LaunchStatus*)mirror_dev_ptr;
     if (p.n_pairs == 0) return;
-    if (use_tma) SKY_CUDA_CHECK(launch_kv_transfer_tma(p, src_pool.numel(), ctas, cur_stream()));
-    else SKY_CUDA_CHECK(launch_kv_transfer(p, ctas, cur_stream()));
+    if (use_tma == 1 || (use_tma == 2 && kv_transfer_tma_takes(p, src_pool.numel()))) SKY_CUDA_CHECK(launch_kv_transfer_tma(p, src_pool.numel(), ctas, cur_stream()));
+    else SKY_CUDA_CHECK(launch_kv_transfer(p, ctas_simt > 0 ? ctas_simt : ctas, cur_stream()));
 }
 
 // ---- causal prefill attention over the paged pool ----
@@ -475,8 +505,10 @@ static void step_increment(torch::Tensor step) {
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     m.doc() = "SkyGDR-B200 sm_100a kernels";
     m.def("new_status", &new_status);
+    m.def("new_flow_work", &new_flow_work);
     m.def("reset_status", &reset_status);
     m.def("read_status", &read_status);
+    m.def("sync_and_read_mirror", &sync_and_read_mirror);
     m.def("host_alloc_mapped", &host_alloc_mapped);
     m.def("host_free_mapped", &host_free_mapped);
     m.def("host_register", &host_register);
@@ -500,8 +532,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
           py::arg("heads"), py::arg("block_tokens"), py::arg("head_dim"), py::arg("src_strides"), py::arg("dst_strides"),
           py::arg("heads_per_dst"), py::arg("replicate"), py::arg("fp8"), py::arg("keep_layout"), py::arg("pages_per_chunk"),
           py::arg("ctas"), py::arg("credit_dev_ptr"), py::arg("consumed_base"), py::arg("max_wait_ns"), py::arg("first_chunk"),
-          py::arg("done_value"), py::arg("status"), py::arg("use_tma"), py::arg("multicast_ptr") = 0,
-          py::arg("src_num_blocks") = 0, py::arg("dst_num_blocks") = 0);
+          py::arg("done_value"), py::arg("status"), py::arg("use_tma"), py::arg("work"), py::arg("mirror_dev_ptr"),
+          py::arg("ctas_simt") = 0, py::arg("multicast_ptr") = 0, py::arg("src_num_blocks") = 0, py::arg("dst_num_blocks") = 0);
     m.def("multicast_supported", [](int device) {
         std::string why;
         bool ok = multicast_supported(device, &why);

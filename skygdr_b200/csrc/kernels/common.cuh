@@ -40,6 +40,11 @@ __device__ __forceinline__ unsigned int ld_acquire_sys_u32(const unsigned int* p
 __device__ __forceinline__ void st_release_sys_u32(unsigned int* p, unsigned int v) {
     asm volatile("st.release.sys.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
+__device__ __forceinline__ ulonglong2 ld_sys_u64x2(const unsigned long long* p) {
+    ulonglong2 v;
+    asm volatile("ld.volatile.global.v2.u64 {%0,%1}, [%2];" : "=l"(v.x), "=l"(v.y) : "l"(p) : "memory");
+    return v;
+}
 __device__ __forceinline__ void st_sys_u64(unsigned long long* p, unsigned long long v) {
     asm volatile("st.relaxed.sys.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
@@ -110,11 +115,14 @@ __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.lau
 // cached in *cache so that an unpaced or generously paced flow touches host
 // memory only once in a while. Returns false when the deadline passed or the
 // page's stop flag is set (then *stopped tells which).
+// With `shared`, whatever is read of the grant is also left in that block in device
+// memory, where the launch's other CTAs find it (KvCredit in kv_transfer.cuh).
 constexpr unsigned long long SKY_UNLIMITED_RECHECK_BYTES = 256ull << 20;
 
 __device__ __forceinline__ bool credit_acquire(const SkyCreditPage* page, unsigned long long need,
                                                unsigned long long* cache, unsigned long long max_wait_ns,
-                                               unsigned long long* stall_ns, bool* stopped, bool* control_lost = nullptr) {
+                                               unsigned long long* stall_ns, bool* stopped, bool* control_lost = nullptr,
+                                               SkyGrantCache* shared = nullptr) {
     *stopped = false;
     if (control_lost) *control_lost = false;
     if (page == nullptr) return true;
@@ -122,23 +130,34 @@ __device__ __forceinline__ bool credit_acquire(const SkyCreditPage* page, unsign
     unsigned long long t0 = globaltimer_ns();
     unsigned ns = 64;
     // Heartbeat: the control side bumps `epoch` every window. If it stays put for dead_after_windows windows while this
-    // thread is waiting for credit, the control side is taken for dead and the page's dead_policy applies.
-    const unsigned dead_windows = ld_sys_u32(&page->dead_after_windows);
-    const unsigned long long dead_ns = dead_windows ? (unsigned long long)dead_windows * ld_sys_u64((const unsigned long long*)&page->window_ns) : 0ull;
-    unsigned long long epoch0 = dead_ns ? ld_sys_u64((const unsigned long long*)&page->epoch) : 0ull, t_epoch = t0, t_dead = 0;
-    // An earlier wait (this CTA's or another's) may have found the heartbeat stale at this very epoch already.
-    bool dead = dead_ns && ld_sys_u64((const unsigned long long*)&page->heartbeat_lost) == epoch0 + 1;
-    if (dead) t_dead = ld_sys_u64((const unsigned long long*)&page->heartbeat_lost_ns);
+    // thread is waiting for credit, the control side is taken for dead and the page's dead_policy applies. Nothing of it is
+    // read before the first look at the grant has failed: every read of the page is a round trip to host memory.
+    bool armed = false, dead = false;
+    unsigned long long dead_ns = 0, epoch0 = 0, t_epoch = t0, t_dead = 0;
     for (;;) {
-        if (ld_sys_u32(&page->stop)) { *stopped = true; *stall_ns += globaltimer_ns() - t0; return false; }
+        // every read of the page costs about 0.7 us, also when it overlaps others: none more than the answer needs
+        const unsigned stop = ld_sys_u32(&page->stop), unl = ld_sys_u32(&page->unlimited);
+        if (stop) { *stopped = true; *stall_ns += globaltimer_ns() - t0; return false; }
         // "unlimited" is not cached for the rest of the launch: the control side may start pacing this flow at any window, and a
         // launch can last many windows. The page is read again after SKY_UNLIMITED_RECHECK_BYTES more of the flow's bytes
         // (a fraction of a millisecond at link rate), which costs an unpaced flow one host-memory read per few chunks per CTA.
-        if (ld_sys_u32(&page->unlimited)) { *cache = need + SKY_UNLIMITED_RECHECK_BYTES; break; }
-        unsigned long long g = ld_sys_u64((const unsigned long long*)&page->granted_bytes);
+        if (unl) { *cache = need + SKY_UNLIMITED_RECHECK_BYTES; if (shared) { shared->unlimited = 1; __threadfence(); atomicMax(&shared->granted, *cache); } break; }
+        const unsigned long long g = ld_sys_u64((const unsigned long long*)&page->granted_bytes);
         *cache = g;
+        if (shared) { shared->unlimited = 0; __threadfence(); atomicMax(&shared->granted, g); }
         if (need <= g) break;
         const unsigned long long now = globaltimer_ns();
+        if (!armed) {
+            armed = true;
+            const unsigned dead_windows = ld_sys_u32(&page->dead_after_windows);
+            dead_ns = dead_windows ? (unsigned long long)dead_windows * ld_sys_u64((const unsigned long long*)&page->window_ns) : 0ull;
+            if (dead_ns) {
+                epoch0 = ld_sys_u64((const unsigned long long*)&page->epoch);
+                // An earlier wait (this CTA's or another's) may have found the heartbeat stale at this very epoch already.
+                dead = ld_sys_u64((const unsigned long long*)&page->heartbeat_lost) == epoch0 + 1;
+                if (dead) t_dead = ld_sys_u64((const unsigned long long*)&page->heartbeat_lost_ns);
+            }
+        }
         if (dead_ns) {
             const unsigned long long e = ld_sys_u64((const unsigned long long*)&page->epoch);
             if (e != epoch0) { epoch0 = e; t_epoch = now; dead = false; }
@@ -152,7 +171,7 @@ __device__ __forceinline__ bool credit_acquire(const SkyCreditPage* page, unsign
             if (dead) {
                 if (control_lost) *control_lost = true;
                 const unsigned policy = ld_sys_u32(&page->dead_policy);
-                if (policy == SKY_DEAD_UNPACED) { *cache = ~0ull; break; }
+                if (policy == SKY_DEAD_UNPACED) { *cache = ~0ull; if (shared) atomicMax(&shared->granted, ~0ull); break; }
                 if (policy == SKY_DEAD_STATIC) {
                     const unsigned long long w = max(1ull, ld_sys_u64((const unsigned long long*)&page->window_ns));
                     const unsigned long long self = g + (now > t_dead ? (now - t_dead) / w : 0ull) * ld_sys_u64((const unsigned long long*)&page->fallback_per_window);

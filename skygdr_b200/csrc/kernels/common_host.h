@@ -18,4 +18,18 @@ struct LaunchStatus {
     unsigned int work_counter;      // dynamic chunk scheduler
 };
 
+// What the CTAs of a launch know of their flow's credit page, in device memory behind the working status block. Reads of the page
+// itself are round trips to host memory that do not overlap (they name the same line): one CTA at a time reads it, for all.
+struct SkyGrantCache {
+    unsigned long long granted;     // largest grant read so far (0: none yet)
+    unsigned int unlimited;         // the last read found the flow unpaced
+    unsigned int lock;              // 1: some CTA is reading the page, or waiting for credit on behalf of all
+};
+
+// Working block of a flow's transfer launches: status, then grant cache.
+struct FlowWork {
+    LaunchStatus status;
+    SkyGrantCache grant;
+};
+
 }  // namespace sky

@@ -17,7 +17,7 @@ from typing import Dict, List, Optional, Sequence
 import torch
 
 from .._ext import load
-from .flow import CreditPage, new_status, read_status
+from .flow import STATUS_NAMES, CreditPage, new_status, read_status
 from .kv_cache import KVGeometry, PagedKVPool
 
 
@@ -127,15 +127,21 @@ class FanoutTarget:
 class KvTransferFlow:
     def __init__(self, device, page: Optional[CreditPage] = None, ctas: Optional[int] = None, pages_per_chunk: int = 8,
                  max_wait_ms: float = 2.0, method: str = "auto"):
-        """method: "tma" (copy hardware does gather, layout change and peer write; bf16 only), "simt" (register path; also
-        fp8 packing and same-layout copies), or "auto" (tma whenever it applies)."""
+        """method: "tma" (copy hardware does gather, layout change and peer write), "simt" (register path; any layout, multicast
+        destinations), or "auto" (tma whenever it applies)."""
         assert method in ("auto", "tma", "simt")
         self.method = method
         self._ctas_given = ctas is not None
         self._C = load()
         self.device = torch.device(device)
+        self._index = self.device.index if self.device.index is not None else torch.cuda.current_device()
         self.page = page
         self.status = new_status(self.device)
+        # A launch counts in a working block that its last CTA leaves reset for the next launch; the outcome goes to ``status``
+        # and to a copy in mapped host memory. So neither a transfer nor its result costs a copy between host and device.
+        self._work = self._C.new_flow_work(self._index)
+        self._mirror_host, self._mirror_dev = self._C.host_alloc_mapped(self._C.STATUS_BYTES)
+        self._launched = False
         self.consumed = 0
         sms = torch.cuda.get_device_properties(self.device).multi_processor_count
         self.sms = sms
@@ -157,27 +163,44 @@ class KvTransferFlow:
         for d in dsts:
             assert replicate or keep_layout or d.kv_heads == heads_per_dst, "destination head count does not match the scatter"
         assert not multicast_ptr or (replicate and not fp8 and not keep_layout), "multicast fan-out carries replicated bf16 pages"
-        use_tma = self.method != "simt" and not multicast_ptr and not fp8 and not keep_layout and g.kv_heads <= 8 and g.head_dim == 128 and src.data.is_contiguous()
-        assert use_tma or self.method != "tma", "the TMA variant moves contiguous bf16 pools of <= 8 heads without fp8 packing"
-        if use_tma and ctas is None and not self._ctas_given:
-            ctas = self.sms                      # one driving thread and a 192 KB ring per SM
+        use_tma = self.method != "simt" and not multicast_ptr and g.kv_heads <= 8 and g.head_dim == 128 and src.data.is_contiguous()
+        assert use_tma or self.method != "tma", "the TMA variant moves contiguous pools of <= 8 heads, to unicast destinations"
+        if use_tma and self.method != "tma":
+            use_tma = 2                          # the extension looks at strides and addresses, and may still take the register path
+        # the copy-hardware engines hold a 192 KB ring per CTA: one per SM
+        n_ctas, n_simt = (self.sms, self.ctas) if ctas is None and not self._ctas_given else (ctas or self.ctas,) * 2
         self.seq += 1
-        self._C.reset_status(self.status)
+        self._launched = src_blocks.numel() > 0
+        if not self._launched:                   # an empty transfer launches nothing: its outcome is a fresh block
+            self._C.reset_status(self.status)
         self._C.kv_transfer(
             src.data, [d.ptr for d in dsts], [d.scale_ptr for d in dsts], [d.done_flag_ptr if signal else 0 for d in dsts],
             src_blocks, dst_blocks, g.layers, g.kv_heads, g.block_tokens, g.head_dim, list(src.strides), list(dsts[0].strides),
-            heads_per_dst, replicate, fp8, keep_layout, self.pages_per_chunk, ctas or self.ctas,
+            heads_per_dst, replicate, fp8, keep_layout, self.pages_per_chunk, n_ctas,
             self.page.dev_ptr if self.page else 0, self.consumed, self.max_wait_ns, first_chunk, self.seq, self.status, use_tma,
-            multicast_ptr=multicast_ptr, src_num_blocks=src.num_blocks, dst_num_blocks=min(d.num_blocks for d in dsts))
+            work=self._work, mirror_dev_ptr=self._mirror_dev, ctas_simt=n_simt, multicast_ptr=multicast_ptr, src_num_blocks=src.num_blocks, dst_num_blocks=min(d.num_blocks for d in dsts))
         self._last = (src, dsts, src_blocks, dst_blocks, replicate, fp8, keep_layout, ctas, multicast_ptr)
 
     def result(self) -> Dict[str, int]:
         """Synchronises and returns the status block; accounts the bytes that were moved."""
-        torch.cuda.synchronize(self.device)
-        st = read_status(self.status)
+        if self._launched:
+            st = self._C.sync_and_read_mirror(self._index, self._mirror_host)
+            st["status_name"] = STATUS_NAMES.get(st["status"], str(st["status"]))
+        else:
+            torch.cuda.synchronize(self.device)
+            st = read_status(self.status)
         self.consumed += st["bytes_done"]
         st["device_time_ms"] = (st["t_end_ns"] - st["t_start_ns"]) * 1e-6 if st["t_end_ns"] else float("nan")
         return st
+
+    def __del__(self):
+        try:
+            if self._mirror_host:
+                torch.cuda.synchronize(self.device)          # a launch may still be about to write the copy
+                self._C.host_free_mapped(self._mirror_host)
+                self._mirror_host = 0
+        except Exception:
+            pass
 
     def resume(self, st: Dict[str, int]) -> None:
         """Relaunches the last transfer from the cursor a yielded launch left behind."""
