@@ -502,7 +502,10 @@ static void step_increment(torch::Tensor step) {
     SKY_CUDA_CHECK(launch_step_increment(reinterpret_cast<unsigned int*>(step.data_ptr()), cur_stream()));
 }
 
+void bind_decoder_stack(py::module_& m);
+
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
+    bind_decoder_stack(m);
     m.doc() = "SkyGDR-B200 sm_100a kernels";
     m.def("new_status", &new_status);
     m.def("new_flow_work", &new_flow_work);

@@ -37,13 +37,8 @@ __device__ __forceinline__ float block_sum(float v, float* red) {
 }
 
 // One CTA per row; each thread owns up to 4 vectors of 8 elements (hidden <= 256*8*4 = 8192).
-__global__ void __launch_bounds__(256) rmsnorm_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* residual,
-                                                       const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ y,
-                                                       int hidden, float eps) {
-    __shared__ float red[8];
-    pdl_trigger();
-    pdl_wait();
-    const long long row = blockIdx.x;
+__device__ __forceinline__ void rmsnorm_row(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* residual, const __nv_bfloat16* __restrict__ w,
+                                            __nv_bfloat16* __restrict__ y, int hidden, float eps, float* red) {
     const int nvec = hidden / 8;
     float vals[4][8];
     float ss = 0.f;
@@ -51,14 +46,14 @@ __global__ void __launch_bounds__(256) rmsnorm_kernel(const __nv_bfloat16* __res
     for (int k = 0; k < 4; ++k) {
         const int v = threadIdx.x + k * 256;
         if (v < nvec) {
-            unpack8(*reinterpret_cast<const uint4*>(x + row * hidden + v * 8), vals[k]);
+            unpack8(*reinterpret_cast<const uint4*>(x + v * 8), vals[k]);
             if (residual) {
                 float r[8];
-                unpack8(*reinterpret_cast<const uint4*>(residual + row * hidden + v * 8), r);
+                unpack8(*reinterpret_cast<const uint4*>(residual + v * 8), r);
 #pragma unroll
                 for (int i = 0; i < 8; ++i) vals[k][i] += r[i];
                 uint4 packed = pack8(vals[k]);
-                *reinterpret_cast<uint4*>(residual + row * hidden + v * 8) = packed;
+                *reinterpret_cast<uint4*>(residual + v * 8) = packed;
                 unpack8(packed, vals[k]);  // normalise what was stored (bf16-rounded), as a two-kernel version would
             }
 #pragma unroll
@@ -75,15 +70,74 @@ __global__ void __launch_bounds__(256) rmsnorm_kernel(const __nv_bfloat16* __res
             unpack8(*reinterpret_cast<const uint4*>(w + v * 8), g);
 #pragma unroll
             for (int i = 0; i < 8; ++i) o[i] = vals[k][i] * inv * g[i];
-            *reinterpret_cast<uint4*>(y + row * hidden + v * 8) = pack8(o);
+            *reinterpret_cast<uint4*>(y + v * 8) = pack8(o);
         }
     }
+}
+
+__global__ void __launch_bounds__(256) rmsnorm_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* residual,
+                                                       const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ y,
+                                                       int hidden, float eps) {
+    __shared__ float red[8];
+    pdl_trigger();
+    pdl_wait();
+    const long long at = (long long)blockIdx.x * hidden;
+    rmsnorm_row(x + at, residual ? residual + at : nullptr, w, y + at, hidden, eps, red);
 }
 
 cudaError_t launch_rmsnorm(const __nv_bfloat16* x, __nv_bfloat16* residual, const __nv_bfloat16* w, __nv_bfloat16* y,
                            int rows, int hidden, float eps, cudaStream_t stream) {
     if (hidden % 8 || hidden > 8192 || rows <= 0) return cudaErrorInvalidValue;
     return launch_pdl(rmsnorm_kernel, dim3(rows), dim3(256), 0, stream, x, residual, w, y, hidden, eps);
+}
+
+__global__ void __launch_bounds__(256) rmsnorm_rows_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* residual,
+                                                            const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ y,
+                                                            const __grid_constant__ RowMap rows, int hidden, float eps) {
+    __shared__ float red[8];
+    pdl_trigger();
+    pdl_wait();
+    const long long from = (long long)rows.src[blockIdx.x] * hidden, to = (long long)rows.dst[blockIdx.x] * hidden;
+    rmsnorm_row(x + from, residual + from, w, y + to, hidden, eps, red);
+}
+
+cudaError_t launch_rmsnorm_rows(const __nv_bfloat16* x, __nv_bfloat16* residual, const __nv_bfloat16* w, __nv_bfloat16* y,
+                                const RowMap& rows, int hidden, float eps, cudaStream_t stream) {
+    if (hidden % 8 || hidden > 8192 || rows.n <= 0 || rows.n > ROW_MAP_MAX) return cudaErrorInvalidValue;
+    return launch_pdl(rmsnorm_rows_kernel, dim3(rows.n), dim3(256), 0, stream, x, residual, w, y, rows, hidden, eps);
+}
+
+// One CTA per token of the pieces. Bound: the copy of the embedding rows (8 KB each at hidden 4096).
+__global__ void __launch_bounds__(128) prefill_setup_kernel(const PrefillSetup p, const __grid_constant__ PrefillPieces pc) {
+    pdl_trigger();
+    pdl_wait();
+    const int tok = pc.tok0[0] + blockIdx.x;
+    int lo = 0, hi = pc.n - 1;                              // the piece that holds this token
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (pc.tok0[mid] <= tok) lo = mid; else hi = mid - 1;
+    }
+    const int off = tok - pc.tok0[lo];
+    const long long at = (long long)pc.src[lo] + off;
+    int id = p.ids64 ? (int)reinterpret_cast<const long long*>(p.ids)[at] : reinterpret_cast<const int*>(p.ids)[at];
+    id = id < 0 ? 0 : (id >= p.vocab ? p.vocab - 1 : id);
+    if (threadIdx.x == 0) {
+        p.positions[tok] = pc.pos0[lo] + off;
+        p.tok_rows[tok] = pc.row[lo];
+        if (off == 0) {
+            p.seq_start[pc.first + lo] = tok;
+            p.pos0[pc.first + lo] = pc.pos0[lo];
+            p.rows[pc.first + lo] = pc.row[lo];
+            if (lo == pc.n - 1) p.seq_start[pc.first + pc.n] = pc.tok0[pc.n];
+        }
+    }
+    for (int v = threadIdx.x; v < p.hidden / 8; v += 128)
+        *reinterpret_cast<uint4*>(p.resid + (long long)tok * p.hidden + v * 8) = *reinterpret_cast<const uint4*>(p.table + (long long)id * p.hidden + v * 8);
+}
+
+cudaError_t launch_prefill_setup(const PrefillSetup& p, const PrefillPieces& pieces, cudaStream_t stream) {
+    if (pieces.n < 1 || pieces.n > PREFILL_PIECES_MAX || p.hidden % 8 || pieces.tok0[pieces.n] <= pieces.tok0[0]) return cudaErrorInvalidValue;
+    return launch_pdl(prefill_setup_kernel, dim3(pieces.tok0[pieces.n] - pieces.tok0[0]), dim3(128), 0, stream, p, pieces);
 }
 
 // One warp per (token, head) over q heads, k heads and v heads; lane owns dims [4*lane, 4*lane+4).

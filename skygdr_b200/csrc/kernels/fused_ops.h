@@ -9,6 +9,31 @@ namespace sky {
 cudaError_t launch_rmsnorm(const __nv_bfloat16* x, __nv_bfloat16* residual, const __nv_bfloat16* w, __nv_bfloat16* y,
                            int rows, int hidden, float eps, cudaStream_t stream);
 
+// y[dst[i]] = rmsnorm(residual[src[i]] + x[src[i]]) * w for a few rows (the last tokens of prompts); residual is updated as above.
+constexpr int ROW_MAP_MAX = 256;
+struct RowMap { int n; int src[ROW_MAP_MAX], dst[ROW_MAP_MAX]; };
+cudaError_t launch_rmsnorm_rows(const __nv_bfloat16* x, __nv_bfloat16* residual, const __nv_bfloat16* w, __nv_bfloat16* y,
+                                const RowMap& rows, int hidden, float eps, cudaStream_t stream);
+
+// The start of a prefill pass: pieces of prompts packed back to back. One launch gathers the embedding rows of their tokens and writes
+// what the later kernels of the pass index by: position and block-table row of every token, and offsets, preceding tokens and
+// block-table row of every piece. The pieces travel as kernel arguments (no copy to the device).
+constexpr int PREFILL_PIECES_MAX = 128;
+struct PrefillPieces {
+    int n, first;                                      // pieces of this launch, and the index of the first of them in the pass
+    int tok0[PREFILL_PIECES_MAX + 1];                  // offset of each piece in the pass, and the end of the last
+    int src[PREFILL_PIECES_MAX];                       // its first token in ids
+    int pos0[PREFILL_PIECES_MAX], row[PREFILL_PIECES_MAX];
+};
+struct PrefillSetup {
+    const void* ids; int ids64;
+    const __nv_bfloat16* table; int vocab, hidden;
+    __nv_bfloat16* resid;                              // [tokens of the pass][hidden]
+    int *positions, *tok_rows;                         // [tokens of the pass]
+    int *seq_start, *pos0, *rows;                      // [pieces + 1], [pieces], [pieces]
+};
+cudaError_t launch_prefill_setup(const PrefillSetup& p, const PrefillPieces& pieces, cudaStream_t stream);
+
 struct RopeAppendParams {
     const __nv_bfloat16* qkv;      // [tokens][(q_heads + 2*kv_heads) * 128]
     const __nv_bfloat16* q_norm;   // [128] or nullptr

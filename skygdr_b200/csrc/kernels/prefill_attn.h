@@ -25,6 +25,7 @@ struct PrefillAttnParams {
     float scale;
     const int* pos0;             // [n_seqs] or nullptr: tokens of each sequence that precede its queries of this launch; their K/V are in
                                  // the pool already and every query attends to them (chunked prefill)
+    const int* seq_rows;         // [n_seqs] or nullptr: row of block_table of each sequence (nullptr: row i belongs to sequence i)
     LaunchStatus* status;
     int page_box;                // set by the launcher: 1 = the K/V map fetches a whole page per request (see prefill_attn_tc.cu)
 };

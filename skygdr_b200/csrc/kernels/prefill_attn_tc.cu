@@ -83,7 +83,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_attn_tc_kernel(const __
     }
     const int n_kt = max(nkt_x[0], nkt_x[1]);
     const int kvh = head / (p.q_heads / p.kv_heads);
-    const int* table = p.block_table + (long long)seq * p.max_blocks;
+    const int* table = p.block_table + (long long)(p.seq_rows ? p.seq_rows[seq] : seq) * p.max_blocks;
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < PF_UNITS; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }

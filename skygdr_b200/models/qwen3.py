@@ -14,12 +14,14 @@ built on this package's own kernels.
 from __future__ import annotations
 
 import math
+import operator
 from dataclasses import dataclass
 from typing import List, Optional
 
 import torch
 
 from .. import ops
+from .._ext import load
 from ..ops.kv_cache import KVGeometry, PagedKVPool
 
 
@@ -176,6 +178,7 @@ class Qwen3Decoder:
         # Set before capture(): a captured graph keeps the choice it was captured with.
         self.temperature, self.sample_seed = 0.0, 0
         self._prefill_attn = None
+        self._stack, self._stack_weights = None, None
         dev = pool.data.device
         self.device = dev
         self.max_batch, self.max_ctx = max_batch, max_ctx
@@ -313,6 +316,49 @@ class Qwen3Decoder:
             passes.append(cur)
         return passes
 
+    def _layer_stack(self):
+        """The layer stack behind the C++ driver (csrc/kernels/decoder_stack.cpp), over the weights as they are now; None where some
+        weight is not in the layout it takes (a strided view), which leaves the op-by-op path below."""
+        w = self.w
+        now = [getattr(lw, k) for lw in w.layers for k in ("qkv", "o", "gate_up", "down", "ln1", "ln2", "q_norm", "k_norm")] + [w.embed, w.final_norm]
+        held = self._stack_weights
+        if held is None or len(held) != len(now) or not all(map(operator.is_, held, now)):
+            fits = bool(w.layers) and all(t.is_cuda and t.dtype == torch.bfloat16 and t.is_contiguous() for t in now)
+            self._stack = load().DecoderStack([now[i:i + 8] for i in range(0, len(now) - 2, 8)], w.embed, w.final_norm, self.inv_freq, self.cfg.q_heads,
+                                              self.cfg.kv_heads, self.cfg.ffn, self.cfg.eps) if fits else None
+            self._stack_weights = now
+        return self._stack
+
+    def _prefill_native(self, stack, ids: torch.Tensor, seq_lens: List[int], block_table: torch.Tensor, pool: PagedKVPool, chunk: int) -> torch.Tensor:
+        from ..ops.gemm import _sms, plan, workspace_for
+
+        cfg, C = self.cfg, load()
+        assert all(n >= 1 for n in seq_lens), "a prompt holds at least one token"
+        if self._prefill_attn is None:
+            self._prefill_attn = ops.PrefillAttention(ids.device)
+        starts, o = [], 0
+        for n in seq_lens:
+            starts.append(o)
+            o += n
+        passes = self.prefill_plan(seq_lens, chunk)
+        sms, ws = _sms(ids.device), workspace_for(ids.device)
+        qkv_cols = (cfg.q_heads + 2 * cfg.kv_heads) * cfg.head_dim
+        shapes = ((qkv_cols, cfg.hidden, False), (cfg.hidden, cfg.q_heads * cfg.head_dim, False), (cfg.ffn, cfg.hidden, True), (cfg.hidden, cfg.ffn, False))
+        choices = []
+        for pieces in passes:
+            T = sum(e - b for _, b, e in pieces)
+            choices.append([plan(T, N, K, sms, gated) for N, K, gated in shapes])
+            for (N, K, gated), (ntok, splits, cluster, _) in zip(shapes, choices[-1]):
+                if splits > 1 and not cluster:
+                    ws.ensure(C.gemm_workspace_floats(T, N, splits, gated, ntok), C.gemm_counter_count(T, N, gated, ntok))
+        s = pool.data.stride()
+        head, tok = (s[3], s[4]) if pool.layout == "hnd" else (s[4], s[3])
+        if ids.dtype not in (torch.int64, torch.int32) or not ids.is_contiguous():
+            ids = ids.int().contiguous()
+        xn = stack.prefill(ids, starts, seq_lens, passes, choices, block_table.contiguous(), pool.data, [s[0], s[1], s[2], head, tok], ws.ws, ws.counters,
+                           ws.status, self._prefill_attn.status)
+        return ops.gemm(xn, self.w.lm_head)
+
     @torch.no_grad()
     def prefill(self, ids: torch.Tensor, seq_lens: List[int], block_table: torch.Tensor, pool: Optional[PagedKVPool] = None,
                 chunk: int = 8192, attn: Optional[str] = None) -> torch.Tensor:
@@ -330,6 +376,10 @@ class Qwen3Decoder:
         pool = pool or self.pool
         dev = ids.device
         D = cfg.head_dim
+        if attn == "tc" and ids.is_cuda:
+            stack = self._layer_stack()
+            if stack is not None:
+                return self._prefill_native(stack, ids, [int(n) for n in seq_lens], block_table, pool, int(chunk))
         starts = [0]
         for n in seq_lens[:-1]:
             starts.append(starts[-1] + int(n))

@@ -2,6 +2,7 @@
 from __future__ import annotations
 
 from dataclasses import dataclass
+from functools import lru_cache
 from typing import Dict, Optional, Tuple
 
 import torch
@@ -67,8 +68,10 @@ def tuned_config(M: int, N: int, K: int, gated: bool) -> Optional[Tuple[int, int
     return (int(e[0]), int(e[1]), bool(e[2])) if e else None
 
 
+@lru_cache(maxsize=4096)
 def choose_config(M: int, N: int, K: int, sms: int, gated: bool = False) -> Tuple[int, int, bool]:
-    """(token tile, splits, cluster) for a decode GEMM: the measured best where the shape was tuned, the cost model otherwise."""
+    """(token tile, splits, cluster) for a decode GEMM: the measured best where the shape was tuned, the cost model otherwise. Kept per
+    shape: the model walks some eighty candidates, 70 us of Python, longer than most of the kernels it chooses for."""
     t = tuned_config(M, N, K, gated)
     if t:
         return t
@@ -121,12 +124,15 @@ class GemmWorkspace:
         self.ws = torch.empty(0, dtype=torch.float32, device=self.device)
         self.counters = torch.zeros(4096, dtype=torch.int32, device=self.device)
         self.status = new_status(self.device)
+        self._outgrown = []          # captured graphs may still name a buffer that has become too small; doubling keeps these few
 
     def ensure(self, floats: int, counters: int):
         if self.ws.numel() < floats:
-            self.ws = torch.empty(floats, dtype=torch.float32, device=self.device)
+            self._outgrown.append(self.ws)
+            self.ws = torch.empty(max(floats, 2 * self.ws.numel()), dtype=torch.float32, device=self.device)
         if self.counters.numel() < counters:
-            self.counters = torch.zeros(counters, dtype=torch.int32, device=self.device)
+            self._outgrown.append(self.counters)
+            self.counters = torch.zeros(max(counters, 2 * self.counters.numel()), dtype=torch.int32, device=self.device)
 
 
 _WS: Dict[int, GemmWorkspace] = {}
@@ -160,6 +166,16 @@ def wide_tiles_pay(M: int, N: int, K: int, sms: int, gated: bool, ntok: int = 0)
 
     speedup = 1.2 / (1.0 + 0.07 * 4096.0 / K)
     return speedup * fill(wide) > fill(narrow)
+
+
+def plan(M: int, N: int, K: int, sms: int, gated: bool = False) -> Tuple[int, int, int, int]:
+    """(token tile, splits, cluster, persistent form: 0 none, 1 narrow, 2 wide) that ``gemm`` takes for this shape when the caller
+    leaves the choice open."""
+    if M > 256:
+        wide = wide_tiles_pay(M, N, K, sms, gated)
+        return (256 if wide else 128 if gated else 256), 1, 0, 2 if wide else 1
+    ntok, splits, cluster = choose_config(M, N, K, sms, gated)
+    return ntok, splits, int(cluster and splits > 1), 0
 
 
 def gemm(x: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = None, gated: bool = False,
