@@ -12,8 +12,10 @@
 #include <vector>
 
 #include "common_host.h"
+#include "decode_gemm.h"
 #include "fused_ops.h"
 #include "gemm_tcgen05.h"
+#include "paged_attn.h"
 #include "prefill_attn.h"
 
 namespace py = pybind11;
@@ -156,6 +158,80 @@ public:
         return out;
     }
 
+    // One decode step of the first `rows` slots up to the logits: an embedding gather, per layer QKV, attention, O, gate/up and down with the
+    // norms, the rotary embedding and the cache append in their epilogues (decode_gemm.cu), and the output projection.
+    //   splits: K slices of the five projections (QKV, O, gate/up, down, output), 0 = by the rule of decode_gemm.cu.
+    void decode(int rows, torch::Tensor ids, torch::Tensor positions, torch::Tensor ctx_lens, torch::Tensor block_table, torch::Tensor resid, torch::Tensor xg,
+                torch::Tensor ss, torch::Tensor q, torch::Tensor ao, torch::Tensor act, torch::Tensor lm_head, torch::Tensor logits, torch::Tensor pool,
+                std::vector<int64_t> strides, int max_ctx, int chunk_tokens, bool tensor_cores, torch::Tensor part_o, torch::Tensor part_m, torch::Tensor part_l,
+                torch::Tensor counters, torch::Tensor attn_status, torch::Tensor gemm_status, std::vector<int> splits) {
+        c10::cuda::CUDAGuard guard(embed_.device());
+        auto stream = at::cuda::getCurrentCUDAStream().stream();
+        const int sms = at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
+        TORCH_CHECK(rows >= 1 && rows <= DECODE_GEMM_MAX_ROWS && hidden_ % 128 == 0 && splits.size() == 5 && strides.size() == 4, "decode: up to 256 rows, hidden a multiple of 128");
+        for (auto& t : {ids, positions, ctx_lens, block_table}) TORCH_CHECK(t.is_cuda() && t.scalar_type() == torch::kInt32 && t.is_contiguous(), "indexes: contiguous CUDA int32");
+        for (auto& t : {resid, xg, q, ao, act, logits, lm_head}) TORCH_CHECK(t.is_cuda() && t.scalar_type() == torch::kBFloat16 && t.is_contiguous(), "activations: contiguous CUDA bf16");
+        TORCH_CHECK(resid.size(0) >= rows && xg.size(0) >= rows && q.size(0) >= rows && ao.size(0) >= rows && act.size(0) >= rows && logits.size(0) >= rows &&
+                    ids.numel() >= rows && positions.numel() >= rows && ctx_lens.numel() >= rows && block_table.size(0) >= rows, "buffers smaller than the batch");
+        TORCH_CHECK(lm_head.size(1) == hidden_ && logits.size(1) == lm_head.size(0) && resid.size(1) == hidden_ && act.size(1) == ffn_, "shapes");
+        const int tiles = hidden_ / 128, pitch = (int)ss.size(1);
+        TORCH_CHECK(ss.is_cuda() && ss.scalar_type() == torch::kFloat32 && ss.is_contiguous() && ss.size(0) >= 2 * tiles && pitch >= rows, "ss: two blocks of hidden / 128 rows");
+        TORCH_CHECK((int64_t)max_ctx <= block_table.size(1) * 16, "max_ctx = ", max_ctx, " but a block-table row covers ", block_table.size(1) * 16, " tokens");
+        const int max_splits = (int)part_m.size(2);
+        TORCH_CHECK(part_o.numel() >= (int64_t)rows * q_heads_ * max_splits * 128 && counters.numel() >= (int64_t)rows * kv_heads_, "attention scratch too small");
+        float* ss_attn = ss.data_ptr<float>();                   // of the row that QKV and the output projection read
+        float* ss_mlp = ss_attn + (int64_t)tiles * pitch;        // of the row that gate/up reads
+
+        DecodeGemmParams base;
+        memset(&base, 0, sizeof base);
+        base.M = rows; base.ss_pitch = pitch; base.norm_dim = hidden_; base.eps = eps_;
+        base.status = reinterpret_cast<LaunchStatus*>(gemm_status.data_ptr());
+        auto project = [&](DecodeGemmParams& p, const __nv_bfloat16* x, const torch::Tensor& w, int N, int K, int which, bool gated) {
+            p.x = x; p.w = bf(w); p.N = N; p.K = K; p.gated = gated;
+            p.splits = splits[which] > 0 ? splits[which] : decode_gemm_splits(rows, N, K, gated, sms);
+            STACK_CHECK(launch_decode_gemm(p, stream));
+        };
+        STACK_CHECK(launch_embed_norm(ids.data_ptr<int>(), bf(embed_), (int)embed_.size(0), hidden_, rows, bf(layers_[0].ln1), bf(resid), bf(xg), ss_attn, stream));
+        int n_ss = 1;
+        for (size_t li = 0; li < layers_.size(); ++li) {
+            const Layer& l = layers_[li];
+            const __nv_bfloat16* layer_base = bf(pool) + (int64_t)li * strides[1];
+            DecodeGemmParams p = base;
+            p.mode = DG_QKV; p.ss_in = ss_attn; p.n_ss = n_ss;
+            RopeAppendParams& r = p.rope;
+            r.q_norm = bf(l.q_norm); r.k_norm = bf(l.k_norm); r.q_out = bf(q); r.kv = const_cast<__nv_bfloat16*>(layer_base);
+            r.inv_freq = inv_freq_.data_ptr<float>(); r.block_table = block_table.data_ptr<int>(); r.positions = positions.data_ptr<int>();
+            r.block_stride = strides[0]; r.kv_stride = strides[2]; r.head_stride = strides[3]; r.tok_stride = 128;
+            r.tokens = rows; r.q_heads = q_heads_; r.kv_heads = kv_heads_; r.max_blocks = (int)block_table.size(1); r.block_tokens = 16; r.eps = eps_;
+            project(p, bf(xg), l.qkv, qkv_cols_, hidden_, 0, false);
+
+            PagedAttnParams a;
+            memset(&a, 0, sizeof a);
+            a.q = bf(q); a.kv = layer_base; a.out = bf(ao); a.block_table = r.block_table; a.ctx_lens = ctx_lens.data_ptr<int>();
+            a.block_stride = strides[0]; a.kv_stride = strides[2]; a.head_stride = strides[3];
+            a.batch = rows; a.q_heads = q_heads_; a.kv_heads = kv_heads_; a.head_dim = 128; a.block_tokens = 16; a.max_blocks = r.max_blocks;
+            a.num_blocks = (int)pool.size(0); a.max_ctx = max_ctx; a.chunk_tokens = chunk_tokens; a.scale = 1.0f / std::sqrt(128.0f); a.max_splits = max_splits;
+            a.part_o = part_o.data_ptr<float>(); a.part_m = part_m.data_ptr<float>(); a.part_l = part_l.data_ptr<float>();
+            a.counters = reinterpret_cast<unsigned int*>(counters.data_ptr());
+            a.status = reinterpret_cast<LaunchStatus*>(attn_status.data_ptr());
+            STACK_CHECK(tensor_cores ? launch_paged_attn_decode_tc(a, (pool.numel() - (int64_t)li * strides[1]) / 128, stream) : launch_paged_attn_decode(a, stream));
+
+            p = base;
+            p.mode = DG_RESID; p.resid = bf(resid); p.xg = bf(xg); p.gain = bf(l.ln2); p.ss_out = ss_mlp;
+            project(p, bf(ao), l.o, hidden_, q_heads_ * 128, 1, false);
+            p = base;
+            p.mode = DG_STORE; p.ss_in = ss_mlp; p.n_ss = tiles; p.y = bf(act); p.ldy = ffn_;
+            project(p, bf(xg), l.gate_up, ffn_, hidden_, 2, true);
+            p = base;
+            p.mode = DG_RESID; p.resid = bf(resid); p.xg = bf(xg); p.gain = li + 1 < layers_.size() ? bf(layers_[li + 1].ln1) : bf(final_norm_); p.ss_out = ss_attn;
+            project(p, bf(act), l.down, hidden_, ffn_, 3, false);
+            n_ss = tiles;
+        }
+        DecodeGemmParams p = base;
+        p.mode = DG_STORE; p.ss_in = ss_attn; p.n_ss = n_ss; p.y = bf(logits); p.ldy = logits.size(1);
+        project(p, bf(xg), lm_head, (int)lm_head.size(0), hidden_, 4, false);
+    }
+
 private:
     void gemm(const __nv_bfloat16* x, int M, int K, const torch::Tensor& w, __nv_bfloat16* y, int N, bool gated, const Choice& c,
               const torch::Tensor& workspace, const torch::Tensor& counters, const torch::Tensor& status, cudaStream_t stream) {
@@ -187,5 +263,10 @@ void bind_decoder_stack(py::module_& m) {
              py::arg("embed"), py::arg("final_norm"), py::arg("inv_freq"), py::arg("q_heads"), py::arg("kv_heads"), py::arg("ffn"), py::arg("eps"))
         .def("prefill", &DecoderStack::prefill, py::call_guard<py::gil_scoped_release>(), py::arg("ids"), py::arg("starts"), py::arg("lens"), py::arg("passes"),
              py::arg("choices"), py::arg("block_table"), py::arg("pool"), py::arg("strides"), py::arg("workspace"), py::arg("counters"),
-             py::arg("gemm_status"), py::arg("attn_status"));
+             py::arg("gemm_status"), py::arg("attn_status"))
+        .def("decode", &DecoderStack::decode, py::call_guard<py::gil_scoped_release>(), py::arg("rows"), py::arg("ids"), py::arg("positions"),
+             py::arg("ctx_lens"), py::arg("block_table"), py::arg("resid"), py::arg("xg"), py::arg("ss"), py::arg("q"), py::arg("ao"), py::arg("act"),
+             py::arg("lm_head"), py::arg("logits"), py::arg("pool"), py::arg("strides"), py::arg("max_ctx"), py::arg("chunk_tokens"),
+             py::arg("tensor_cores"), py::arg("part_o"), py::arg("part_m"), py::arg("part_l"), py::arg("counters"), py::arg("attn_status"),
+             py::arg("gemm_status"), py::arg("splits"));
 }

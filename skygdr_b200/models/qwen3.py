@@ -179,6 +179,7 @@ class Qwen3Decoder:
         self.temperature, self.sample_seed = 0.0, 0
         self._prefill_attn = None
         self._stack, self._stack_weights = None, None
+        self._decode_splits = [0] * 5
         dev = pool.data.device
         self.device = dev
         self.max_batch, self.max_ctx = max_batch, max_ctx
@@ -200,9 +201,22 @@ class Qwen3Decoder:
         self.block_table = torch.zeros((B, self.max_blocks), dtype=torch.int32, device=dev)
         self.inv_freq = ops.rope_inv_freq(cfg.rope_theta, dev, cfg.head_dim)
         self.attn = ops.PagedAttention(dev, B, cfg.q_heads, cfg.kv_heads, max_ctx, attn_chunk, impl=attn_impl)
+        self.ss = torch.empty((2 * max(1, cfg.hidden // 128), B), dtype=torch.float32, device=dev)   # partial sums of squares of the residual rows
         self.graph: Optional[torch.cuda.CUDAGraph] = None
         self.graph_batch = 0
-        self.kernels_per_step = 1 + 8 * cfg.layers + 3   # embedding, 8 per layer, final norm, lm_head, argmax
+
+    @property
+    def kernels_per_step(self) -> int:
+        if self._decode_stack(self.max_batch) is not None:
+            return 1 + 5 * self.cfg.layers + 2           # embedding, 5 per layer, lm_head, argmax
+        return 1 + 8 * self.cfg.layers + 3               # embedding, 8 per layer, final norm, lm_head, argmax
+
+    def _decode_stack(self, b: int):
+        """The C++ driver of the fused step (csrc/kernels/decode_gemm.cu), or None where it does not take the model or the batch."""
+        cfg = self.cfg
+        if self.pool.data.device.type != "cuda" or b > 256 or cfg.hidden % 128 or cfg.ffn % 64 or not self.w.lm_head.is_contiguous() or not self.pool.data.is_contiguous():
+            return None
+        return self._layer_stack()
 
     # ---- state ----
     def set_batch(self, ids: torch.Tensor, positions: torch.Tensor, block_table: torch.Tensor) -> None:
@@ -216,6 +230,17 @@ class Qwen3Decoder:
 
     # ---- one decode step for the first `b` slots ----
     def _step(self, b: int, max_ctx: int) -> None:
+        stack = self._decode_stack(b)
+        if stack is not None:
+            from ..ops.gemm import workspace_for
+
+            a, s = self.attn, self.pool.data.stride()
+            max_ctx = min(max_ctx, a.max_ctx, self.block_table.shape[1] * 16)
+            stack.decode(b, self.ids, self.positions, self.ctx_lens, self.block_table, self.resid, self.xn, self.ss, self.q, self.attn_out, self.act,
+                         self.w.lm_head, self.logits, self.pool.data, list(s[:4]), max_ctx, a.chunk_tokens, a.impl == "tc", a.part_o, a.part_m, a.part_l,
+                         a.counters, a.status, workspace_for(self.device).status, self._decode_splits)
+            self._pick(b)
+            return
         cfg, w = self.cfg, self.w
         resid, xn, h = self.resid[:b], self.xn[:b], self.h[:b]
         qkv, q, ao, act = self.qkv[:b], self.q[:b], self.attn_out[:b], self.act[:b]
