@@ -16,7 +16,9 @@
 //   * the residual add, and RMSNorm split in two: the epilogue of O and down writes resid * gain and its tile's sums of squares per
 //     row; the next projection multiplies the finished product by the row's 1 / rms (it is linear in x);
 //   * QK-norm, rotary embedding and the append to the paged cache: a tile of the QKV projection is exactly one head.
-// FIGURES
+// One B200, 8 layers of Qwen3-8B's widths, host token ids in and out, against separate kernels on the general projection: one sequence
+// 1061 -> 1008 us, 16 sequences of 2k to 16k tokens 1885 -> 1810 us, 32 of 1k to 32k 3049 -> 2626 us, 100 short ones with sampling
+// 1964 -> 1869 us; prefill of 77 tokens 2174 -> 1118 us (with the passes driven from C++).
 #include <cuda.h>
 
 #include <algorithm>
@@ -36,27 +38,12 @@ constexpr int DG_THREADS = 192;
 constexpr int DG_BM = 128, DG_BK = 64;
 constexpr int DG_W_BYTES = DG_BM * DG_BK * 2;
 constexpr int DG_MAX_STAGES = 8;
-constexpr int DG_PITCH = 132;                      // floats between staged rows of 128 values (16-byte rows, banks shifted)
 
 struct DgShape {                                   // derived on the host once per launch
     int ntok, stages, stage_bytes, acc_cols, tmem_cols;
     int up_col;                                    // first TMEM column (and partial column) of the up accumulator
-    int stage_off;                                 // where finished rows are staged, behind the partials
 };
 
-__device__ __forceinline__ uint32_t dg_ctarank() { uint32_t r; asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r)); return r; }
-__device__ __forceinline__ void dg_cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
-__device__ __forceinline__ void dg_cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
-__device__ __forceinline__ uint32_t dg_peer(uint32_t local, uint32_t rank) {
-    uint32_t a;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(local), "r"(rank));
-    return a;
-}
-__device__ __forceinline__ float dg_ld_peer(uint32_t addr) {
-    float v;
-    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
-    return v;
-}
 __device__ __forceinline__ void epi_bar() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
 __device__ __forceinline__ void unpack4(uint2 v, float* f) {
     f[0] = __uint_as_float(v.x << 16); f[1] = __uint_as_float(v.x & 0xffff0000u);
@@ -68,39 +55,76 @@ __device__ __forceinline__ uint2 pack4(const float* f) {
 }
 __device__ __forceinline__ float silu_mul_f(float g, float u) { return g / (1.0f + __expf(-g)) * u; }
 
-// One finished row of a tile: lane holds columns 4 lane .. 4 lane + 3 of the 128.
-__device__ __forceinline__ void finish_row(const DecodeGemmParams& p, int tile, int t, int lane, float* v, int pos, int blk) {
+// Finished rows t0, t0 + 4, ... (U of them, those below t_end) of a tile: lane holds columns 4 lane .. 4 lane + 3 of the 128. Several rows
+// at once, because a row by itself is a chain of load, shuffles and store.
+template <int MODE, int U>
+__device__ __forceinline__ void finish_rows(const DecodeGemmParams& p, int tile, int t0, int t_end, int lane, float (*v)[4], const int* s_pos, const int* s_blk) {
     const int n0 = tile * DG_BM;
-    if (p.mode == DG_STORE) {
-        const int n = n0 + lane * 4;
-        __nv_bfloat16* dst = p.y + (long long)t * p.ldy + n;
-        if (n + 4 <= p.N && (reinterpret_cast<uintptr_t>(dst) & 7) == 0) *reinterpret_cast<uint2*>(dst) = pack4(v);
-        else
-            for (int i = 0; i < 4 && n + i < p.N; ++i) dst[i] = __float2bfloat16(v[i]);
-    } else if (p.mode == DG_RESID) {
-        const long long at = (long long)t * p.N + n0 + lane * 4;
-        float r[4], g[4];
-        unpack4(*reinterpret_cast<const uint2*>(p.resid + at), r);
+    if (MODE == DG_STORE) {
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int t = t0 + 4 * u, n = n0 + lane * 4;
+            if (t >= t_end) break;
+            __nv_bfloat16* dst = p.y + (long long)t * p.ldy + n;
+            if (n + 4 <= p.N && (reinterpret_cast<uintptr_t>(dst) & 7) == 0) *reinterpret_cast<uint2*>(dst) = pack4(v[u]);
+            else
+                for (int i = 0; i < 4 && n + i < p.N; ++i) dst[i] = __float2bfloat16(v[u][i]);
+        }
+    } else if (MODE == DG_RESID) {
+        const long long at = (long long)t0 * p.N + n0 + lane * 4;
+        uint2 res[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) res[u] = t0 + 4 * u < t_end ? *reinterpret_cast<const uint2*>(p.resid + at + 4LL * u * p.N) : make_uint2(0, 0);
+        float g[4], ss[U];
         unpack4(__ldg(reinterpret_cast<const uint2*>(p.gain + n0 + lane * 4)), g);
 #pragma unroll
-        for (int i = 0; i < 4; ++i) r[i] += v[i];
-        const uint2 packed = pack4(r);
-        *reinterpret_cast<uint2*>(p.resid + at) = packed;
-        unpack4(packed, r);                        // the norm sees what was stored
-        float ss = r[0] * r[0] + r[1] * r[1] + r[2] * r[2] + r[3] * r[3];
+        for (int u = 0; u < U; ++u) {
+            float r[4];
+            unpack4(res[u], r);
 #pragma unroll
-        for (int i = 0; i < 4; ++i) g[i] *= r[i];
-        *reinterpret_cast<uint2*>(p.xg + at) = pack4(g);
-        for (int o = 16; o; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-        if (lane == 0) p.ss_out[(long long)tile * p.ss_pitch + t] = ss;
+            for (int i = 0; i < 4; ++i) r[i] += v[u][i];
+            const uint2 packed = pack4(r);
+            unpack4(packed, r);                    // the norm sees what is stored
+            ss[u] = r[0] * r[0] + r[1] * r[1] + r[2] * r[2] + r[3] * r[3];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) r[i] *= g[i];
+            if (t0 + 4 * u < t_end) {
+                *reinterpret_cast<uint2*>(p.resid + at + 4LL * u * p.N) = packed;
+                *reinterpret_cast<uint2*>(p.xg + at + 4LL * u * p.N) = pack4(r);
+            }
+        }
+#pragma unroll
+        for (int o = 16; o; o >>= 1)
+#pragma unroll
+            for (int u = 0; u < U; ++u) ss[u] += __shfl_xor_sync(0xffffffffu, ss[u], o);
+        if (lane == 0)
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                if (t0 + 4 * u < t_end) p.ss_out[(long long)tile * p.ss_pitch + t0 + 4 * u] = ss[u];
     } else {
-        float cs[4], sn[4];
-        rope_angles(pos, p.rope.inv_freq, lane, cs, sn);
-        rope_append_row(p.rope, t, tile, lane, v, pos, blk, cs, sn);
+        if (p.round_product)
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) v[u][i] = __bfloat162float(__float2bfloat16(v[u][i]));
+        if (tile < p.rope.q_heads + p.rope.kv_heads) {
+            const __nv_bfloat16* weight = tile < p.rope.q_heads ? p.rope.q_norm : p.rope.k_norm;
+            if (weight) rope_norm_rows<U>(weight, p.rope.eps, lane, v);
+            const float4 freqs = rope_freqs(p.rope.inv_freq, lane);
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                float cs[4], sn[4];
+                rope_angles(t0 + 4 * u < t_end ? s_pos[t0 + 4 * u] : 0, freqs, cs, sn);
+                rope_rotate(lane, v[u], cs, sn);
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (t0 + 4 * u < t_end) rope_store(p.rope, t0 + 4 * u, tile, lane, v[u], s_pos[t0 + 4 * u], s_blk[t0 + 4 * u]);
     }
 }
 
-template <bool GATED>
+template <bool GATED, int MODE>
 __global__ void __launch_bounds__(DG_THREADS, 2) decode_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
                                                                      const __grid_constant__ DecodeGemmParams p, const DgShape sh) {
     extern __shared__ unsigned char smem_raw[];
@@ -187,7 +211,6 @@ __global__ void __launch_bounds__(DG_THREADS, 2) decode_gemm_kernel(const __grid
     // ---- epilogue ----
     const int c_lo = split * sh.ntok / splits, c_hi = min((split + 1) * sh.ntok / splits, p.M);      // this CTA's token rows
     float* part = reinterpret_cast<float*>(smem);                        // [acc_cols][128], over the idle ring
-    float* rows = reinterpret_cast<float*>(smem + sh.stage_off);         // [c_hi - c_lo][DG_PITCH]
     const int ew = warp - 2;                                             // 0..3; TMEM lanes 32 (warp % 4) ..
     const int r = (warp & 3) * 32 + lane;                                // weight row inside the tile
     const uint32_t taddr = tmem_base + ((uint32_t)((warp & 3) * 32) << 16);
@@ -205,7 +228,7 @@ __global__ void __launch_bounds__(DG_THREADS, 2) decode_gemm_kernel(const __grid
             }
             if (lane == 0) {
                 s_inv[t] = inv;
-                if (p.mode == DG_QKV) {
+                if (MODE == DG_QKV) {
                     const int pos = p.rope.positions[t];
                     s_pos[t] = pos;
                     s_blk[t] = p.rope.block_table[(long long)(p.rope.seq_ids ? p.rope.seq_ids[t] : t) * p.rope.max_blocks + pos / p.rope.block_tokens];
@@ -215,124 +238,153 @@ __global__ void __launch_bounds__(DG_THREADS, 2) decode_gemm_kernel(const __grid
         if (nkb > 0) ok = mbar_wait(&acc_bar, 0);
         if (!ok && lane == 0) set_status(p.status, SKY_STATUS_TIMEOUT_MBAR, 83);
         tc_fence_after();
-        if (splits > 1) {
-            for (int c = 0; c < sh.acc_cols; c += 16) {
+        // the accumulator, token column by token column, to shared memory; a gated tile that is not split is finished on the way
+        if (GATED && splits == 1) {
+            epi_bar();                                                   // s_inv is written
+            for (int c = 0; c < sh.ntok; c += 16) {
+                uint32_t v[16], u[16];
+                tmem_ld_x16(taddr + c, v);
+                tmem_ld_x16(taddr + sh.up_col + c, u);
+                tc_wait_ld();
+#pragma unroll
+                for (int i = 0; i < 16; ++i) {
+                    const float inv = c + i < p.M ? s_inv[c + i] : 0.f;
+                    part[(c + i) * DG_BM + r] = ok ? silu_mul_f(__uint_as_float(v[i]) * inv, __uint_as_float(u[i]) * inv) : 0.f;
+                }
+            }
+        } else {
+            int c = 0;
+            for (; c + 32 <= sh.acc_cols; c += 32) {
+                uint32_t v[32];
+                tmem_ld_x32(taddr + c, v);
+                tc_wait_ld();
+#pragma unroll
+                for (int i = 0; i < 32; ++i) part[(c + i) * DG_BM + r] = ok ? __uint_as_float(v[i]) : 0.f;
+            }
+            if (c < sh.acc_cols) {
                 uint32_t v[16];
                 tmem_ld_x16(taddr + c, v);
                 tc_wait_ld();
 #pragma unroll
                 for (int i = 0; i < 16; ++i) part[(c + i) * DG_BM + r] = ok ? __uint_as_float(v[i]) : 0.f;
             }
-        } else {
-            for (int c = 0; c < c_hi; c += 16) {
-                uint32_t v[16], u[16];
-                tmem_ld_x16(taddr + c, v);
-                if (GATED) tmem_ld_x16(taddr + sh.up_col + c, u);
-                tc_wait_ld();
-                epi_bar();                                               // s_inv is written; and the staged rows of the last round have been read
-#pragma unroll
-                for (int i = 0; i < 16; ++i) {
-                    if (c + i >= c_hi) break;
-                    const float inv = s_inv[c + i];
-                    float val = __uint_as_float(v[i]) * inv;
-                    if (GATED) val = silu_mul_f(val, __uint_as_float(u[i]) * inv);
-                    rows[i * DG_PITCH + r] = ok ? val : 0.f;
-                }
-                epi_bar();
-                for (int t = c + ew; t < min(c + 16, c_hi); t += 4) {
-                    float4 q = *reinterpret_cast<const float4*>(rows + (t - c) * DG_PITCH + lane * 4);
-                    finish_row(p, tile, t, lane, reinterpret_cast<float*>(&q), s_pos[t], s_blk[t]);
-                }
-            }
         }
     }
     if (splits > 1) {
         tc_fence_before();
-        dg_cluster_arrive();
-        dg_cluster_wait();                                               // every CTA's partial is in its shared memory
-        if (warp >= 2) {
-            uint32_t peer[8];
+        cluster_arrive();
+        cluster_wait();                                                  // every CTA's partial is in its shared memory
+    }
+    if (warp >= 2) {
+        if (splits == 1) epi_bar();
+        constexpr int U = GATED ? 2 : 4;                                 // rows at once: their loads from all slices are in flight together
+        const uint32_t own = smem_u32(part) + (uint32_t)lane * 16u;
+        for (int t0 = c_lo + ew; t0 < c_hi; t0 += 4 * U) {
+            float v[U][4];
+            if (splits == 1) {
 #pragma unroll
-            for (int s = 0; s < 8; ++s) peer[s] = s < splits ? dg_peer(smem_u32(smem), (uint32_t)s) + (uint32_t)r * 4u : 0u;
-            constexpr int CH = 4;                                        // columns per round: 4 x splits loads in flight (gated: twice)
-            for (int c = c_lo; c < c_hi; c += CH) {
-                float g[CH] = {}, u[CH] = {};
+                for (int u = 0; u < U; ++u) {
+                    const int t = t0 + 4 * u;
+                    const float4 q = t < c_hi ? *reinterpret_cast<const float4*>(part + t * DG_BM + lane * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
+                    const float inv = GATED || t >= c_hi ? 1.0f : s_inv[t];
+                    v[u][0] = q.x * inv; v[u][1] = q.y * inv; v[u][2] = q.z * inv; v[u][3] = q.w * inv;
+                }
+            } else {
+                float up[U][4];
 #pragma unroll
-                for (int half = 0; half < (GATED ? 2 : 1); ++half) {
-                    float a[8][CH];
+                for (int u = 0; u < U; ++u)
 #pragma unroll
-                    for (int s = 0; s < 8; ++s)
+                    for (int i = 0; i < 4; ++i) v[u][i] = up[u][i] = 0.f;
+                for (int s0 = 0; s0 < splits; s0 += 4) {
+                    float4 a[4][U], b[4][U];
 #pragma unroll
-                        for (int i = 0; i < CH; ++i)
-                            a[s][i] = (s < splits && c + i < c_hi) ? dg_ld_peer(peer[s] + (uint32_t)((half * sh.up_col + c + i) * DG_BM) * 4u) : 0.f;
+                    for (int s = 0; s < 4; ++s) {
+                        const uint32_t peer = dsmem_addr(own, (uint32_t)min(s0 + s, splits - 1));
 #pragma unroll
-                    for (int s = 0; s < 8; ++s)
+                        for (int u = 0; u < U; ++u) {
+                            const int t = t0 + 4 * u;
+                            const bool in = s0 + s < splits && t < c_hi;
+                            a[s][u] = in ? ld_dsmem_f32x4(peer + (uint32_t)(t * DG_BM) * 4u) : make_float4(0.f, 0.f, 0.f, 0.f);
+                            if (GATED) b[s][u] = in ? ld_dsmem_f32x4(peer + (uint32_t)((sh.up_col + t) * DG_BM) * 4u) : make_float4(0.f, 0.f, 0.f, 0.f);
+                        }
+                    }
 #pragma unroll
-                        for (int i = 0; i < CH; ++i) (half ? u : g)[i] += a[s][i];
+                    for (int s = 0; s < 4; ++s)
+#pragma unroll
+                        for (int u = 0; u < U; ++u) {
+                            v[u][0] += a[s][u].x; v[u][1] += a[s][u].y; v[u][2] += a[s][u].z; v[u][3] += a[s][u].w;
+                            if (GATED) { up[u][0] += b[s][u].x; up[u][1] += b[s][u].y; up[u][2] += b[s][u].z; up[u][3] += b[s][u].w; }
+                        }
                 }
 #pragma unroll
-                for (int i = 0; i < CH; ++i)
-                    if (c + i < c_hi) {
-                        const float inv = s_inv[c + i];
-                        rows[(c + i - c_lo) * DG_PITCH + r] = GATED ? silu_mul_f(g[i] * inv, u[i] * inv) : g[i] * inv;
-                    }
+                for (int u = 0; u < U; ++u) {
+                    const float inv = t0 + 4 * u < c_hi ? s_inv[t0 + 4 * u] : 1.0f;
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) v[u][i] = GATED ? silu_mul_f(v[u][i] * inv, up[u][i] * inv) : v[u][i] * inv;
+                }
             }
+            finish_rows<MODE, U>(p, tile, t0, c_hi, lane, v, s_pos, s_blk);
         }
-        dg_cluster_arrive();                                             // this CTA has read its peers
-        if (warp >= 2) {
-            epi_bar();
-            for (int t = c_lo + ew; t < c_hi; t += 4) {
-                float4 q = *reinterpret_cast<const float4*>(rows + (t - c_lo) * DG_PITCH + lane * 4);
-                finish_row(p, tile, t, lane, reinterpret_cast<float*>(&q), s_pos[t], s_blk[t]);
-            }
-        }
+    }
+    if (splits > 1) {
         __syncwarp();
-        dg_cluster_wait();                                               // and nobody reads this one any more
+        cluster_arrive();
+        cluster_wait();                                                  // nobody reads this CTA's shared memory any more
     }
     tc_fence_before();
     __syncthreads();
     if (warp == 1) tmem_dealloc(tmem_base, (uint32_t)sh.tmem_cols);
 }
 
+// Token and accumulator columns of a launch.
+DgShape dg_cols(int M, bool gated) {
+    DgShape sh = {};
+    sh.ntok = (M + 15) / 16 * 16;
+    sh.up_col = (sh.ntok + 31) / 32 * 32;
+    sh.acc_cols = gated ? sh.up_col + sh.ntok : sh.ntok;
+    return sh;
+}
+// Shared memory of the finished or partial columns, over the ring.
+int part_bytes(const DgShape& sh, int splits) { return (splits > 1 ? sh.acc_cols : sh.ntok) * DG_BM * 4; }
+constexpr int DG_MAX_BYTES = 217 * 1024;           // of 227 KB, less the alignment of the ring and the static part
+
 }  // namespace
 
 // Splits of K per tile: as many as bring the launch to about one CTA per SM (a CTA then leaves room for one of the next kernel, which
 // streams its first weight tiles meanwhile), at most 8 (a portable cluster) and at least 4 k-blocks each.
+// The fp32 partials of a slice have to fit in shared memory: a gated tile of more than some 200 tokens does not split.
 int decode_gemm_splits(int M, int N, int K, bool gated, int sms) {
     const int tiles = (N + DG_BM - 1) / DG_BM, kb = K / DG_BK;
-    int s = std::max(1, std::min({8, sms / tiles, kb / 4}));
-    return s;
+    const int s = std::max(1, std::min({8, sms / tiles, kb / 4}));
+    return s > 1 && part_bytes(dg_cols(M, gated), s) > DG_MAX_BYTES ? 1 : s;
 }
 
 cudaError_t launch_decode_gemm(const DecodeGemmParams& p, cudaStream_t stream) {
     if (p.M < 1 || p.M > DECODE_GEMM_MAX_ROWS || p.N < 1 || p.K < DG_BK || p.K % DG_BK || p.splits < 1 || p.splits > 8 || p.splits > p.K / DG_BK) return cudaErrorInvalidValue;
     if (p.mode != DG_STORE && (p.N % DG_BM || p.gated)) return cudaErrorInvalidValue;
     if (p.mode == DG_QKV && p.N != (p.rope.q_heads + 2 * p.rope.kv_heads) * 128) return cudaErrorInvalidValue;
-    DgShape sh;
-    sh.ntok = (p.M + 15) / 16 * 16;
-    sh.up_col = (sh.ntok + 31) / 32 * 32;
-    sh.acc_cols = p.gated ? sh.up_col + sh.ntok : sh.ntok;
+    DgShape sh = dg_cols(p.M, p.gated);
     sh.tmem_cols = 32;
     while (sh.tmem_cols < sh.acc_cols) sh.tmem_cols *= 2;
     sh.stage_bytes = DG_W_BYTES * (p.gated ? 2 : 1) + sh.ntok * DG_BK * 2;
-    const int part = p.splits > 1 ? sh.acc_cols * DG_BM * 4 : 0;
-    sh.stage_off = part;
-    const int rows = (p.splits > 1 ? (sh.ntok + p.splits - 1) / p.splits + 1 : 16) * DG_PITCH * 4;
+    const int part = part_bytes(sh, p.splits);
     // Two CTAs per SM (this kernel's and the next one's, or two of a launch with many tiles) where three stages fit in half of the
     // shared memory and half of TMEM is enough; one otherwise. With one, no second CTA can wait for TMEM that it will not get.
-    const bool two = 3 * sh.stage_bytes <= 104 * 1024 && part + rows <= 104 * 1024 && sh.tmem_cols <= 256;
+    const bool two = 3 * sh.stage_bytes <= 104 * 1024 && part <= 104 * 1024 && sh.tmem_cols <= 256;
     const int budget = two ? 104 * 1024 : 200 * 1024;
     sh.stages = std::min(DG_MAX_STAGES, budget / sh.stage_bytes);
-    int bytes = std::max(sh.stages * sh.stage_bytes, part + rows);
+    int bytes = std::max(sh.stages * sh.stage_bytes, part);
     if (!two) bytes = std::max(bytes, 116 * 1024);
-    if (bytes > 226 * 1024 - 1024 - 8 * 1024 || sh.stages < 2) return cudaErrorInvalidValue;
+    if (bytes > DG_MAX_BYTES || sh.stages < 2) return cudaErrorInvalidValue;
     bytes += 1024;
     CUtensorMap tw, tx;
     if (!make_tmap_bf16_2d(&tw, p.w, p.gated ? 2LL * p.N : p.N, p.K, p.K, DG_BM)) return cudaErrorInvalidValue;
     if (!make_tmap_bf16_2d(&tx, p.x, p.M, p.K, p.K, sh.ntok)) return cudaErrorInvalidValue;
-    static unsigned long long attr_mask[2] = {0, 0};
-    auto kern = p.gated ? decode_gemm_kernel<true> : decode_gemm_kernel<false>;
-    if (cudaError_t e = set_max_dynamic_smem_once(reinterpret_cast<const void*>(kern), 218 * 1024, &attr_mask[p.gated ? 1 : 0]); e != cudaSuccess) return e;
+    static unsigned long long attr_mask[4] = {0, 0, 0, 0};
+    const int form = p.gated ? 3 : p.mode;
+    auto kern = p.gated ? decode_gemm_kernel<true, DG_STORE> : p.mode == DG_STORE ? decode_gemm_kernel<false, DG_STORE>
+                        : p.mode == DG_RESID ? decode_gemm_kernel<false, DG_RESID> : decode_gemm_kernel<false, DG_QKV>;
+    if (cudaError_t e = set_max_dynamic_smem_once(reinterpret_cast<const void*>(kern), 218 * 1024, &attr_mask[form]); e != cudaSuccess) return e;
     return launch_pdl_cluster(kern, dim3((p.N + DG_BM - 1) / DG_BM, 1, p.splits), dim3(DG_THREADS), (size_t)bytes, stream, p.splits, tw, tx, p, sh);
 }
 

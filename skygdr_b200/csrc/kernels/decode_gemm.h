@@ -37,6 +37,7 @@ struct DecodeGemmParams {
     float* ss_out;               // [N / 128][ss_pitch]
     // DG_QKV (N = (q_heads + 2 kv_heads) * 128)
     RopeAppendParams rope;       // qkv is not used
+    int round_product;           // round the product to bf16 before the norm, as a projection that stores it would
     LaunchStatus* status;
 };
 

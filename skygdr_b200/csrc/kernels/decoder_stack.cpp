@@ -96,6 +96,7 @@ public:
         int* seq_start = tok_rows + most;
         int* pos0 = seq_start + pieces_most + 1;
         int* rows = pos0 + pieces_most;
+        const int sms = at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
         PrefillSetup setup{ids.data_ptr(), ids.scalar_type() == torch::kInt64, bf(embed_), (int)embed_.size(0), hidden_, bf(resid), positions, tok_rows, seq_start, pos0, rows};
 
         for (size_t i = 0; i < passes.size(); ++i) {
@@ -116,19 +117,14 @@ public:
                 }
             }
             if (T == 0) continue;
-            TORCH_CHECK(choices[i].size() == 4, "a choice for each of the four projections");
-            for (size_t li = 0; li < layers_.size(); ++li) {
-                const Layer& l = layers_[li];
-                STACK_CHECK(launch_rmsnorm(li ? bf(h) : bf(resid), li ? bf(resid) : nullptr, bf(l.ln1), bf(xn), T, hidden_, eps_, stream));
-                gemm(bf(xn), T, hidden_, l.qkv, bf(qkv), qkv_cols_, false, choices[i][0], workspace, counters, gemm_status, stream);
-                RopeAppendParams r;
-                memset(&r, 0, sizeof r);
+            RopeAppendParams r;
+            memset(&r, 0, sizeof r);
+            r.qkv = bf(qkv); r.q_out = bf(q);
+            r.inv_freq = inv_freq_.data_ptr<float>(); r.block_table = block_table.data_ptr<int>(); r.positions = positions; r.seq_ids = tok_rows;
+            r.block_stride = strides[0]; r.kv_stride = strides[2]; r.head_stride = strides[3]; r.tok_stride = strides[4];
+            r.tokens = T; r.q_heads = q_heads_; r.kv_heads = kv_heads_; r.max_blocks = (int)block_table.size(1); r.block_tokens = 16; r.eps = eps_;
+            auto attention = [&](size_t li) {
                 const __nv_bfloat16* layer_base = bf(pool) + (int64_t)li * strides[1];
-                r.qkv = bf(qkv); r.q_norm = bf(l.q_norm); r.k_norm = bf(l.k_norm); r.q_out = bf(q); r.kv = const_cast<__nv_bfloat16*>(layer_base);
-                r.inv_freq = inv_freq_.data_ptr<float>(); r.block_table = block_table.data_ptr<int>(); r.positions = positions; r.seq_ids = tok_rows;
-                r.block_stride = strides[0]; r.kv_stride = strides[2]; r.head_stride = strides[3]; r.tok_stride = strides[4];
-                r.tokens = T; r.q_heads = q_heads_; r.kv_heads = kv_heads_; r.max_blocks = (int)block_table.size(1); r.block_tokens = 16; r.eps = eps_;
-                STACK_CHECK(launch_rope_append(r, stream));
                 PrefillAttnParams a;
                 memset(&a, 0, sizeof a);
                 a.q = bf(q); a.kv = layer_base; a.out = bf(ao); a.block_table = block_table.data_ptr<int>(); a.seq_start = seq_start;
@@ -137,10 +133,37 @@ public:
                 a.max_len = longest; a.total_tokens = T; a.scale = 1.0f / std::sqrt(128.0f); a.pos0 = pos0; a.seq_rows = rows;
                 a.status = reinterpret_cast<LaunchStatus*>(attn_status.data_ptr());
                 STACK_CHECK(launch_prefill_attn_tc(a, (pool.numel() - (int64_t)li * strides[1]) / 128, stream));
-                gemm(bf(ao), T, q_heads_ * 128, l.o, bf(h), hidden_, false, choices[i][1], workspace, counters, gemm_status, stream);
+            };
+            // Passes of few tokens take the projections of a decode step: QK-norm, rotary embedding and cache append in the epilogue of QKV.
+            // The norms stay kernels of their own here: with them in the epilogues too (16 launches of 3 us less at 8 layers) the
+            // rounding of every projection's input differs from the longer passes', and K and V of one prompt should not
+            // depend on how it was cut into passes.
+            const bool few = T <= DECODE_GEMM_MAX_ROWS && hidden_ % 64 == 0 && ffn_ % 64 == 0;
+            auto status = reinterpret_cast<LaunchStatus*>(gemm_status.data_ptr());
+            TORCH_CHECK(choices[i].size() == 4, "a choice for each of the four projections");
+            auto projection = [&](const __nv_bfloat16* x, const torch::Tensor& w, __nv_bfloat16* y, int N, int K, bool gated, int which) {
+                if (!few) return gemm(x, T, K, w, y, N, gated, choices[i][which], workspace, counters, gemm_status, stream);
+                DecodeGemmParams p = project_base(T, 0, status);
+                p.mode = DG_STORE; p.y = y; p.ldy = N;
+                project(p, x, w, N, K, 0, gated, sms, stream);
+            };
+            for (size_t li = 0; li < layers_.size(); ++li) {
+                const Layer& l = layers_[li];
+                STACK_CHECK(launch_rmsnorm(li ? bf(h) : bf(resid), li ? bf(resid) : nullptr, bf(l.ln1), bf(xn), T, hidden_, eps_, stream));
+                r.q_norm = bf(l.q_norm); r.k_norm = bf(l.k_norm); r.kv = bf(pool) + (int64_t)li * strides[1];
+                if (few) {
+                    DecodeGemmParams p = project_base(T, 0, status);
+                    p.mode = DG_QKV; p.rope = r; p.round_product = 1;
+                    project(p, bf(xn), l.qkv, qkv_cols_, hidden_, 0, false, sms, stream);
+                } else {
+                    projection(bf(xn), l.qkv, bf(qkv), qkv_cols_, hidden_, false, 0);
+                    STACK_CHECK(launch_rope_append(r, stream));
+                }
+                attention(li);
+                projection(bf(ao), l.o, bf(h), hidden_, q_heads_ * 128, false, 1);
                 STACK_CHECK(launch_rmsnorm(bf(h), bf(resid), bf(l.ln2), bf(xn), T, hidden_, eps_, stream));
-                gemm(bf(xn), T, hidden_, l.gate_up, bf(act), ffn_, true, choices[i][2], workspace, counters, gemm_status, stream);
-                gemm(bf(act), T, ffn_, l.down, bf(h), hidden_, false, choices[i][3], workspace, counters, gemm_status, stream);
+                projection(bf(xn), l.gate_up, bf(act), ffn_, hidden_, true, 2);
+                projection(bf(act), l.down, bf(h), hidden_, ffn_, false, 3);
             }
             RowMap rm;                                     // prompts that end in this pass: their last row, normed
             rm.n = 0;
@@ -179,35 +202,19 @@ public:
         TORCH_CHECK((int64_t)max_ctx <= block_table.size(1) * 16, "max_ctx = ", max_ctx, " but a block-table row covers ", block_table.size(1) * 16, " tokens");
         const int max_splits = (int)part_m.size(2);
         TORCH_CHECK(part_o.numel() >= (int64_t)rows * q_heads_ * max_splits * 128 && counters.numel() >= (int64_t)rows * kv_heads_, "attention scratch too small");
-        float* ss_attn = ss.data_ptr<float>();                   // of the row that QKV and the output projection read
-        float* ss_mlp = ss_attn + (int64_t)tiles * pitch;        // of the row that gate/up reads
-
-        DecodeGemmParams base;
-        memset(&base, 0, sizeof base);
-        base.M = rows; base.ss_pitch = pitch; base.norm_dim = hidden_; base.eps = eps_;
-        base.status = reinterpret_cast<LaunchStatus*>(gemm_status.data_ptr());
-        auto project = [&](DecodeGemmParams& p, const __nv_bfloat16* x, const torch::Tensor& w, int N, int K, int which, bool gated) {
-            p.x = x; p.w = bf(w); p.N = N; p.K = K; p.gated = gated;
-            p.splits = splits[which] > 0 ? splits[which] : decode_gemm_splits(rows, N, K, gated, sms);
-            STACK_CHECK(launch_decode_gemm(p, stream));
-        };
-        STACK_CHECK(launch_embed_norm(ids.data_ptr<int>(), bf(embed_), (int)embed_.size(0), hidden_, rows, bf(layers_[0].ln1), bf(resid), bf(xg), ss_attn, stream));
-        int n_ss = 1;
-        for (size_t li = 0; li < layers_.size(); ++li) {
-            const Layer& l = layers_[li];
-            const __nv_bfloat16* layer_base = bf(pool) + (int64_t)li * strides[1];
-            DecodeGemmParams p = base;
-            p.mode = DG_QKV; p.ss_in = ss_attn; p.n_ss = n_ss;
-            RopeAppendParams& r = p.rope;
-            r.q_norm = bf(l.q_norm); r.k_norm = bf(l.k_norm); r.q_out = bf(q); r.kv = const_cast<__nv_bfloat16*>(layer_base);
-            r.inv_freq = inv_freq_.data_ptr<float>(); r.block_table = block_table.data_ptr<int>(); r.positions = positions.data_ptr<int>();
-            r.block_stride = strides[0]; r.kv_stride = strides[2]; r.head_stride = strides[3]; r.tok_stride = 128;
-            r.tokens = rows; r.q_heads = q_heads_; r.kv_heads = kv_heads_; r.max_blocks = (int)block_table.size(1); r.block_tokens = 16; r.eps = eps_;
-            project(p, bf(xg), l.qkv, qkv_cols_, hidden_, 0, false);
-
+        STACK_CHECK(launch_embed_norm(ids.data_ptr<int>(), bf(embed_), (int)embed_.size(0), hidden_, rows, bf(layers_[0].ln1), bf(resid), bf(xg), ss.data_ptr<float>(), stream));
+        RopeAppendParams r;
+        memset(&r, 0, sizeof r);
+        r.q_out = bf(q);
+        r.inv_freq = inv_freq_.data_ptr<float>(); r.block_table = block_table.data_ptr<int>(); r.positions = positions.data_ptr<int>();
+        r.block_stride = strides[0]; r.kv_stride = strides[2]; r.head_stride = strides[3]; r.tok_stride = 128;
+        r.tokens = rows; r.q_heads = q_heads_; r.kv_heads = kv_heads_; r.max_blocks = (int)block_table.size(1); r.block_tokens = 16; r.eps = eps_;
+        auto status = reinterpret_cast<LaunchStatus*>(gemm_status.data_ptr());
+        FusedRows f{rows, pitch, bf(resid), bf(xg), bf(q), bf(ao), bf(act), ss.data_ptr<float>()};
+        const int n_ss = fused_layers(f, r, bf(pool), strides[1], status, splits, sms, stream, [&](size_t li) {
             PagedAttnParams a;
             memset(&a, 0, sizeof a);
-            a.q = bf(q); a.kv = layer_base; a.out = bf(ao); a.block_table = r.block_table; a.ctx_lens = ctx_lens.data_ptr<int>();
+            a.q = bf(q); a.kv = bf(pool) + (int64_t)li * strides[1]; a.out = bf(ao); a.block_table = r.block_table; a.ctx_lens = ctx_lens.data_ptr<int>();
             a.block_stride = strides[0]; a.kv_stride = strides[2]; a.head_stride = strides[3];
             a.batch = rows; a.q_heads = q_heads_; a.kv_heads = kv_heads_; a.head_dim = 128; a.block_tokens = 16; a.max_blocks = r.max_blocks;
             a.num_blocks = (int)pool.size(0); a.max_ctx = max_ctx; a.chunk_tokens = chunk_tokens; a.scale = 1.0f / std::sqrt(128.0f); a.max_splits = max_splits;
@@ -215,24 +222,56 @@ public:
             a.counters = reinterpret_cast<unsigned int*>(counters.data_ptr());
             a.status = reinterpret_cast<LaunchStatus*>(attn_status.data_ptr());
             STACK_CHECK(tensor_cores ? launch_paged_attn_decode_tc(a, (pool.numel() - (int64_t)li * strides[1]) / 128, stream) : launch_paged_attn_decode(a, stream));
-
-            p = base;
-            p.mode = DG_RESID; p.resid = bf(resid); p.xg = bf(xg); p.gain = bf(l.ln2); p.ss_out = ss_mlp;
-            project(p, bf(ao), l.o, hidden_, q_heads_ * 128, 1, false);
-            p = base;
-            p.mode = DG_STORE; p.ss_in = ss_mlp; p.n_ss = tiles; p.y = bf(act); p.ldy = ffn_;
-            project(p, bf(xg), l.gate_up, ffn_, hidden_, 2, true);
-            p = base;
-            p.mode = DG_RESID; p.resid = bf(resid); p.xg = bf(xg); p.gain = li + 1 < layers_.size() ? bf(layers_[li + 1].ln1) : bf(final_norm_); p.ss_out = ss_attn;
-            project(p, bf(act), l.down, hidden_, ffn_, 3, false);
-            n_ss = tiles;
-        }
-        DecodeGemmParams p = base;
-        p.mode = DG_STORE; p.ss_in = ss_attn; p.n_ss = n_ss; p.y = bf(logits); p.ldy = logits.size(1);
-        project(p, bf(xg), lm_head, (int)lm_head.size(0), hidden_, 4, false);
+        });
+        DecodeGemmParams p = project_base(f.n, f.pitch, status);
+        p.mode = DG_STORE; p.ss_in = f.ss; p.n_ss = n_ss; p.y = bf(logits); p.ldy = logits.size(1);
+        project(p, f.xg, lm_head, (int)lm_head.size(0), hidden_, splits[4], false, sms, stream);
     }
 
 private:
+    // The rows of a pass of at most DECODE_GEMM_MAX_ROWS tokens and the scratch that its layers share. ss: partial sums of squares, [2][hidden / 128]
+    // [pitch]: first those of the rows that QKV and the output projection read, then those that gate/up reads.
+    struct FusedRows { int n, pitch; __nv_bfloat16 *resid, *xg, *q, *ao, *act; float* ss; };
+
+    DecodeGemmParams project_base(int rows, int pitch, LaunchStatus* status) const {
+        DecodeGemmParams p;
+        memset(&p, 0, sizeof p);
+        p.M = rows; p.ss_pitch = pitch; p.norm_dim = hidden_; p.eps = eps_; p.status = status;
+        return p;
+    }
+    void project(DecodeGemmParams& p, const __nv_bfloat16* x, const torch::Tensor& w, int N, int K, int splits, bool gated, int sms, cudaStream_t stream) const {
+        p.x = x; p.w = bf(w); p.N = N; p.K = K; p.gated = gated;
+        p.splits = splits > 0 ? splits : decode_gemm_splits(p.M, N, K, gated, sms);
+        STACK_CHECK(launch_decode_gemm(p, stream));
+    }
+    // All layers over rows whose embedding (resid, and xg = resid * first gain, and one sum of squares per row) is in place; attention(layer)
+    // launches the attention of q into ao. Returns the number of partial sums per row that the output projection finds in f.ss.
+    template <typename Attention>
+    int fused_layers(const FusedRows& f, RopeAppendParams rope, __nv_bfloat16* pool, int64_t layer_stride, LaunchStatus* status, const std::vector<int>& splits,
+                     int sms, cudaStream_t stream, Attention attention) const {
+        const int tiles = hidden_ / 128;
+        float *ss_attn = f.ss, *ss_mlp = f.ss + (int64_t)tiles * f.pitch;
+        for (size_t li = 0; li < layers_.size(); ++li) {
+            const Layer& l = layers_[li];
+            DecodeGemmParams p = project_base(f.n, f.pitch, status);
+            p.mode = DG_QKV; p.ss_in = ss_attn; p.n_ss = li ? tiles : 1;
+            p.rope = rope;
+            p.rope.q_norm = bf(l.q_norm); p.rope.k_norm = bf(l.k_norm); p.rope.kv = pool + (int64_t)li * layer_stride;
+            project(p, f.xg, l.qkv, qkv_cols_, hidden_, splits[0], false, sms, stream);
+            attention(li);
+            p = project_base(f.n, f.pitch, status);
+            p.mode = DG_RESID; p.resid = f.resid; p.xg = f.xg; p.gain = bf(l.ln2); p.ss_out = ss_mlp;
+            project(p, f.ao, l.o, hidden_, q_heads_ * 128, splits[1], false, sms, stream);
+            p = project_base(f.n, f.pitch, status);
+            p.mode = DG_STORE; p.ss_in = ss_mlp; p.n_ss = tiles; p.y = f.act; p.ldy = ffn_;
+            project(p, f.xg, l.gate_up, ffn_, hidden_, splits[2], true, sms, stream);
+            p = project_base(f.n, f.pitch, status);
+            p.mode = DG_RESID; p.resid = f.resid; p.xg = f.xg; p.gain = li + 1 < layers_.size() ? bf(layers_[li + 1].ln1) : bf(final_norm_); p.ss_out = ss_attn;
+            project(p, f.act, l.down, hidden_, ffn_, splits[3], false, sms, stream);
+        }
+        return tiles;
+    }
+
     void gemm(const __nv_bfloat16* x, int M, int K, const torch::Tensor& w, __nv_bfloat16* y, int N, bool gated, const Choice& c,
               const torch::Tensor& workspace, const torch::Tensor& counters, const torch::Tensor& status, cudaStream_t stream) {
         GemmParams p;

@@ -71,23 +71,6 @@ __device__ __forceinline__ void store_chunk16(const GemmParams& p, __nv_bfloat16
     asm volatile("bar.sync %0, 128;" ::"r"(bar) : "memory");
 }
 
-// Thread-block cluster pieces of the split-K form below: the CTAs of one output tile (one per K range) form a cluster and
-// reduce their partial accumulators through each other's shared memory instead of through global memory.
-__device__ __forceinline__ uint32_t cluster_ctarank() { uint32_t r; asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r)); return r; }
-__device__ __forceinline__ void cluster_sync_all() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-__device__ __forceinline__ uint32_t dsmem_addr(uint32_t local_smem_addr, uint32_t cta_rank) {
-    uint32_t a;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(local_smem_addr), "r"(cta_rank));
-    return a;
-}
-__device__ __forceinline__ float ld_dsmem_f32(uint32_t addr) {
-    float v;
-    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
-    return v;
-}
-
 constexpr int GEMM_THREADS = 192;
 constexpr int BM = 128;   // weight rows per tile (MMA M)
 constexpr int BK = 64;    // K per stage: 64 bf16 = 128 bytes = one swizzle row

@@ -102,6 +102,71 @@ def test_graph_replay_equals_eager():
         assert torch.equal(a, b)
 
 
+@pytest.mark.parametrize("b,splits", [(1, 0), (15, 3), (16, 8), (17, 2), (33, 5), (64, 4), (100, 0), (128, 1), (129, 7), (256, 0)])
+def test_fused_decode_step_equals_the_op_by_op_step(b, splits):
+    """The projections with norms, rotary embedding and cache append in their epilogues (csrc/kernels/decode_gemm.cu) against the
+    separate kernels: token counts around the MMA's multiples of 16, every cluster size, uneven slices of K, rows behind the batch."""
+    from skygdr_b200 import ops
+    from skygdr_b200.models import Qwen3Config, Qwen3Decoder, Qwen3Weights
+
+    cfg = Qwen3Config.tiny(layers=2, vocab=1000)                        # 1000: the last tile of the output projection is ragged
+    w = Qwen3Weights(cfg, "cuda", seed=3, std=0.05)
+    cap, g = b + 3, torch.Generator(device="cuda").manual_seed(b)
+    pools = [ops.PagedKVPool(cfg.geometry, 2 * cap + 1, "hnd") for _ in range(2)]
+    pools[0].data.normal_(generator=g)
+    pools[1].data.copy_(pools[0].data)
+    ids = torch.randint(0, cfg.vocab, (b,), device="cuda", generator=g).int()
+    pos = torch.randint(0, 32, (b,), device="cuda", generator=g).int()
+    table = (torch.randperm(2 * cap, device="cuda", generator=g) + 1).int().view(cap, 2)[:b].contiguous()
+    engs = [Qwen3Decoder(cfg, w, pool, max_batch=cap, max_ctx=32, attn_chunk=128) for pool in pools]
+    engs[0]._decode_splits = [splits] * 5
+    assert engs[0]._decode_stack(b) is not None
+    engs[1]._decode_stack = lambda _: None
+    for e in engs:
+        e.logits.fill_(7.0)
+        e.set_batch(ids, pos, table)
+        e.step(b=b, advance=False)
+        assert e.check_status() == "OK"
+    got, want = engs[0].logits[:b].float(), engs[1].logits[:b].float()
+    # Both sides round to bf16 (2^-9 relative at most, 2^-9 / sqrt(3) rms) at nine ops of each layer and four outside: 22 independent
+    # roundings a side add up to 2^-9 sqrt(2 * 22 / 3) = 0.0075 of the norm; twice that for what a layer amplifies.
+    assert ((got - want).norm() / want.norm()).item() < 0.015
+    assert ((pools[0].data.float() - pools[1].data.float()).norm() / pools[1].data.float().norm()).item() < 0.015
+    touched = (pools[0].data != pools[1].data).flatten(1).any(1).nonzero().flatten()
+    assert set(touched.tolist()) <= set(table.flatten().tolist())
+    assert bool((engs[0].logits[b:] == 7.0).all())
+
+
+@pytest.mark.parametrize("lens", [[1], [17, 1, 30], [129], [200, 56], [250, 7], [256, 300]])
+@pytest.mark.parametrize("layout", ["hnd", "nhd"])
+def test_prefill_of_few_tokens_equals_the_op_by_op_prefill(lens, layout):
+    """Passes of up to 256 tokens take the fused projections, longer ones the separate kernels (257 tokens here, and 256 + 300
+    tokens in passes of 300 and 256), in both page layouts; the K and V of the prompts, and only they, are written."""
+    from skygdr_b200 import ops
+    from skygdr_b200.models import Qwen3Config, Qwen3Decoder, Qwen3Weights
+
+    cfg = Qwen3Config.tiny(layers=2, vocab=1000)
+    w = Qwen3Weights(cfg, "cuda", seed=4, std=0.05)
+    g = torch.Generator(device="cuda").manual_seed(sum(lens))
+    ids = torch.randint(0, cfg.vocab, (sum(lens),), device="cuda", generator=g)
+    table = _tables(lens, 24, nblocks=80)
+    out = []
+    for native in (True, False):
+        pool = ops.PagedKVPool(cfg.geometry, 80, layout)
+        pool.data.fill_(300.0)
+        eng = Qwen3Decoder(cfg, w, pool if layout == "hnd" else ops.PagedKVPool(cfg.geometry, 2, "hnd"), max_batch=1, max_ctx=64, attn_chunk=128)
+        if not native:
+            eng._layer_stack = lambda: None
+        logits = eng.prefill(ids, lens, table, pool=pool, chunk=300)
+        assert eng.check_status() == "OK"
+        out.append((logits.float(), pool.data.float()))
+    (got, kv), (want, kv_want) = out
+    assert ((got - want).norm() / want.norm()).item() < 0.015            # as derived for the decode step above
+    assert torch.equal(kv == 300.0, kv_want == 300.0)                     # the same places stay untouched (no K or V is that large)
+    at = kv != 300.0
+    assert ((kv - kv_want)[at].norm() / kv_want[at].norm()).item() < 0.015
+
+
 def test_tensor_parallel_shards_tile_the_full_weights():
     from skygdr_b200.models import Qwen3Config, Qwen3Weights
 
