@@ -222,37 +222,6 @@ cudaError_t launch_embedding(const int* ids, const __nv_bfloat16* table, __nv_bf
     return launch_pdl(embedding_kernel, dim3(tokens), dim3(128), 0, stream, ids, table, out, hidden, vocab);
 }
 
-__global__ void __launch_bounds__(1024) argmax_kernel(const __nv_bfloat16* __restrict__ logits, int* __restrict__ out, int vocab,
-                                                       long long row_stride) {
-    __shared__ float sv[32];
-    __shared__ int si[32];
-    pdl_trigger();
-    pdl_wait();
-    const __nv_bfloat16* row = logits + (long long)blockIdx.x * row_stride;
-    float best = -INFINITY;
-    int bi = 0x7fffffff;
-    for (int c = threadIdx.x; c < vocab; c += 1024) {
-        const float v = __bfloat162float(row[c]);
-        if (v > best || (v == best && c < bi)) { best = v; bi = c; }
-    }
-    for (int o = 16; o; o >>= 1) {
-        const float ov = __shfl_xor_sync(0xffffffffu, best, o);
-        const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-        if (ov > best || (ov == best && oi < bi)) { best = ov; bi = oi; }
-    }
-    if ((threadIdx.x & 31) == 0) { sv[threadIdx.x >> 5] = best; si[threadIdx.x >> 5] = bi; }
-    __syncthreads();
-    if (threadIdx.x < 32) {
-        best = sv[threadIdx.x]; bi = si[threadIdx.x];
-        for (int o = 16; o; o >>= 1) {
-            const float ov = __shfl_xor_sync(0xffffffffu, best, o);
-            const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-            if (ov > best || (ov == best && oi < bi)) { best = ov; bi = oi; }
-        }
-        if (threadIdx.x == 0) out[blockIdx.x] = bi;
-    }
-}
-
 // Temperature sampling without a normalisation pass (Gumbel-max): argmax_c (logit_c / T + g_c) with g_c = -log(-log(u_c)) and
 // u_c uniform in (0, 1) picks column c with probability softmax(logits / T)_c. u_c comes from a counter-based hash of
 // (seed, position of the row's sequence, row, column), so a replayed CUDA graph draws fresh noise every step (the position
@@ -263,49 +232,112 @@ __device__ __forceinline__ unsigned int sample_hash(unsigned int seed, unsigned 
     return h;
 }
 
-__global__ void __launch_bounds__(1024) sample_kernel(const __nv_bfloat16* __restrict__ logits, int* __restrict__ out, int vocab,
-                                                       long long row_stride, float inv_temperature, unsigned int seed,
-                                                       const int* __restrict__ positions) {
-    __shared__ float sv[32];
-    __shared__ int si[32];
+struct Pick { float v; int c; };
+__device__ __forceinline__ void pick_better(Pick& best, float v, int c) {
+    if (v > best.v || (v == best.v && c < best.c)) { best.v = v; best.c = c; }
+}
+__device__ __forceinline__ Pick warp_pick(Pick best) {
+    for (int o = 16; o; o >>= 1) {
+        const float v = __shfl_xor_sync(0xffffffffu, best.v, o);
+        const int c = __shfl_xor_sync(0xffffffffu, best.c, o);
+        pick_better(best, v, c);
+    }
+    return best;
+}
+
+// Column of the largest value of each row (lowest index wins ties), greedy or with the sampling noise added. A row is shared by a
+// cluster of gridDim.z CTAs, each scanning one contiguous span in 16-byte loads; the spans' winners meet in shared memory.
+// Bound: at one row, the latency of the loads (300 KB of logits, just written, out of L2); at a hundred sampled rows the hash and the
+// two logarithms of every column.
+constexpr int PICK_THREADS = 512;
+template <bool SAMPLE>
+__global__ void __launch_bounds__(PICK_THREADS) pick_kernel(const __nv_bfloat16* __restrict__ logits, int* __restrict__ out, int vocab,
+                                                            long long row_stride, float inv_temperature, unsigned int seed, const int* __restrict__ positions) {
+    __shared__ Pick warp_best[PICK_THREADS / 32];
+    __shared__ Pick cta_best;
     pdl_trigger();
     pdl_wait();
-    const __nv_bfloat16* row = logits + (long long)blockIdx.x * row_stride;
-    const unsigned int pos = positions ? (unsigned int)positions[blockIdx.x] : 0u;
-    float best = -INFINITY;
-    int bi = 0x7fffffff;
-    for (int c = threadIdx.x; c < vocab; c += 1024) {
-        const float u = ((float)(sample_hash(seed, pos, blockIdx.x, (unsigned int)c) >> 8) + 0.5f) * (1.0f / 16777216.0f);
-        const float v = __bfloat162float(row[c]) * inv_temperature - logf(-logf(u));
-        if (v > best || (v == best && c < bi)) { best = v; bi = c; }
+    const unsigned int row_id = blockIdx.x;
+    const int splits = (int)gridDim.z, split = (int)blockIdx.z;
+    const __nv_bfloat16* row = logits + (long long)row_id * row_stride;
+    const unsigned int pos = SAMPLE && positions ? (unsigned int)positions[row_id] : 0u;
+    Pick best = {-INFINITY, 0x7fffffff};
+    auto take = [&](float x, int c) {
+        if (SAMPLE) {
+            const float u = ((float)(sample_hash(seed, pos, row_id, (unsigned int)c) >> 8) + 0.5f) * (1.0f / 16777216.0f);
+            x = x * inv_temperature - logf(-logf(u));
+        }
+        pick_better(best, x, c);
+    };
+    if (((reinterpret_cast<uintptr_t>(logits) | (uintptr_t)(row_stride * 2)) & 15) == 0) {
+        const int vecs = vocab / 8;
+        const int lo = (int)((long long)vecs * split / splits), hi = (int)((long long)vecs * (split + 1) / splits);
+        constexpr int DEPTH = SAMPLE ? 2 : 4;               // loads in flight per thread
+        for (int v = lo + threadIdx.x; v < hi; v += DEPTH * PICK_THREADS) {
+            uint4 raw[DEPTH];
+#pragma unroll
+            for (int d = 0; d < DEPTH; ++d)
+                if (v + d * PICK_THREADS < hi) raw[d] = *reinterpret_cast<const uint4*>(row + (long long)(v + d * PICK_THREADS) * 8);
+#pragma unroll
+            for (int d = 0; d < DEPTH; ++d)
+                if (v + d * PICK_THREADS < hi) {
+                    float f[8];
+                    unpack8(raw[d], f);
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) take(f[i], (v + d * PICK_THREADS) * 8 + i);
+                }
+        }
+        if (split == splits - 1)
+            for (int c = vecs * 8 + threadIdx.x; c < vocab; c += PICK_THREADS) take(__bfloat162float(row[c]), c);
+    } else {                                                // rows that start off a 16-byte boundary
+        const int lo = (int)((long long)vocab * split / splits), hi = (int)((long long)vocab * (split + 1) / splits);
+        for (int c = lo + threadIdx.x; c < hi; c += PICK_THREADS) take(__bfloat162float(row[c]), c);
     }
-    for (int o = 16; o; o >>= 1) {
-        const float ov = __shfl_xor_sync(0xffffffffu, best, o);
-        const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-        if (ov > best || (ov == best && oi < bi)) { best = ov; bi = oi; }
-    }
-    if ((threadIdx.x & 31) == 0) { sv[threadIdx.x >> 5] = best; si[threadIdx.x >> 5] = bi; }
+    best = warp_pick(best);
+    if ((threadIdx.x & 31) == 0) warp_best[threadIdx.x >> 5] = best;
     __syncthreads();
     if (threadIdx.x < 32) {
-        best = sv[threadIdx.x]; bi = si[threadIdx.x];
-        for (int o = 16; o; o >>= 1) {
-            const float ov = __shfl_xor_sync(0xffffffffu, best, o);
-            const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-            if (ov > best || (ov == best && oi < bi)) { best = ov; bi = oi; }
+        best = warp_pick(threadIdx.x < PICK_THREADS / 32 ? warp_best[threadIdx.x] : Pick{-INFINITY, 0x7fffffff});
+        if (threadIdx.x == 0) {
+            if (splits == 1) out[row_id] = best.c; else cta_best = best;
         }
-        if (threadIdx.x == 0) out[blockIdx.x] = bi;
     }
+    if (splits == 1) return;
+    cluster_sync_all();
+    if (split == 0 && threadIdx.x < 32) {
+        Pick other = {-INFINITY, 0x7fffffff};
+        if ((int)threadIdx.x < splits) {
+            const uint32_t at = dsmem_addr(smem_u32(&cta_best), threadIdx.x);
+            other.v = ld_dsmem_f32(at);
+            other.c = __float_as_int(ld_dsmem_f32(at + 4));
+        }
+        other = warp_pick(other);
+        if (threadIdx.x == 0) out[row_id] = other.c;
+    }
+    __syncwarp();
+    cluster_sync_all();                                         // nobody leaves while CTA 0 reads
+}
+
+// CTAs per row: as many of 1, 2, 4, 8 as fit the GPU in one wave (four CTAs of 512 threads per SM), and at least 4096 columns each.
+static int pick_splits(int rows, int vocab) {
+    int dev = 0, sms = 148;
+    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    int s = 1;
+    while (s < 8 && (long long)rows * s * 2 <= 4LL * sms && vocab / (s * 2) >= 4096) s *= 2;
+    return s;
 }
 
 cudaError_t launch_sample(const __nv_bfloat16* logits, int* out, int rows, int vocab, long long row_stride, float temperature,
                           unsigned int seed, const int* positions, cudaStream_t stream) {
     if (rows <= 0 || vocab <= 0 || !(temperature > 0.f)) return cudaErrorInvalidValue;
-    return launch_pdl(sample_kernel, dim3(rows), dim3(1024), 0, stream, logits, out, vocab, row_stride, 1.0f / temperature, seed, positions);
+    const int s = pick_splits(rows, vocab);
+    return launch_pdl_cluster(pick_kernel<true>, dim3(rows, 1, s), dim3(PICK_THREADS), 0, stream, s, logits, out, vocab, row_stride, 1.0f / temperature, seed, positions);
 }
 
 cudaError_t launch_argmax(const __nv_bfloat16* logits, int* out, int rows, int vocab, long long row_stride, cudaStream_t stream) {
     if (rows <= 0 || vocab <= 0) return cudaErrorInvalidValue;
-    return launch_pdl(argmax_kernel, dim3(rows), dim3(1024), 0, stream, logits, out, vocab, row_stride);
+    const int s = pick_splits(rows, vocab);
+    return launch_pdl_cluster(pick_kernel<false>, dim3(rows, 1, s), dim3(PICK_THREADS), 0, stream, s, logits, out, vocab, row_stride, 1.0f, 0u, (const int*)nullptr);
 }
 
 }  // namespace sky

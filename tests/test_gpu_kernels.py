@@ -596,6 +596,29 @@ def test_persistent_gemm_with_wide_tiles_matches_reference(ops, M, N, K, gated):
     assert (y.float() - y2.float()).abs().max() < 2e-2 * max(1.0, float(ref.abs().max()))
 
 
+@pytest.mark.parametrize("rows,vocab,pad", [(1, 151936, 0), (5, 32768, 0), (3, 8191, 1), (2, 40004, 4), (75, 16384, 0), (150, 9000, 8), (300, 4099, 5),
+                                            (4, 7, 1), (1, 1, 0)])
+def test_argmax_and_sampling_over_the_ctas_of_a_row(ops, rows, vocab, pad):
+    """One to eight CTAs per row, rows off a 16-byte boundary, widths that are no multiple of a load: the lowest index of the maximum
+    wins wherever the tied columns lie, and values below every finite one are handled as by a plain scan."""
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    full = torch.randint(-50, 50, (rows, vocab + pad), device="cuda", generator=g).bfloat16()     # whole numbers: many ties
+    logits = full[:, :vocab]
+    logits[0] = float("-inf")
+    if rows > 1:
+        logits[1, -1] = 100.0
+    first = torch.tensor([int((row == row.max()).nonzero()[0]) for row in logits.cpu()])
+    assert torch.equal(ops.argmax(logits).cpu().long(), first)
+    if rows > 1 and vocab > 1:
+        drawn = ops.sample(logits[1:], 0.9, seed=5).cpu().long()[:, None]
+        want, v = ops.sample_reference(logits[1:].cpu(), 0.9, 5)
+        # The fast logarithm is off by at most 2^-21.4 in [0.5, 2], which moves noise of size n by 2^-21.4 exp(n); the outer logarithm
+        # and the sum add a few 2^-17 at values up to 64.
+        err = 2.0 ** -21.4 * torch.exp(v - logits[1:].cpu().float() / 0.9) + 5e-5
+        best = want.long()[:, None]
+        assert bool((v.gather(1, drawn) + err.gather(1, drawn) >= v.gather(1, best) - err.gather(1, best)).all())
+
+
 def test_temperature_sampling_matches_the_cpu_restatement(ops):
     """Gumbel-max sampling: the kernel's pick must be the CPU oracle's pick (same hash, fp32 arithmetic), except where the two
     best perturbed values are within rounding of each other; positions change the draw, the seed changes the stream."""
