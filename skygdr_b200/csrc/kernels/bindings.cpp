@@ -381,6 +381,24 @@ static void sample(torch::Tensor logits, torch::Tensor out, double temperature, 
                                  (float)temperature, (unsigned int)seed, pos, cur_stream()));
 }
 
+static void advance(torch::Tensor next_ids, torch::Tensor ids, torch::Tensor positions, torch::Tensor ctx_lens, int64_t n) {
+    c10::cuda::CUDAGuard g(ids.device());
+    for (auto& t : {next_ids, ids, positions, ctx_lens})
+        TORCH_CHECK(t.is_cuda() && t.scalar_type() == torch::kInt32 && t.is_contiguous() && n >= 1 && t.numel() >= n, "state: CUDA int32, at least n entries");
+    SKY_CUDA_CHECK(launch_advance(next_ids.data_ptr<int>(), ids.data_ptr<int>(), positions.data_ptr<int>(), ctx_lens.data_ptr<int>(), (int)n, cur_stream()));
+}
+// False, and nothing done, unless the host tensors are int32 of one length.
+static bool step_inputs(torch::Tensor host_ids, torch::Tensor host_positions, torch::Tensor ids, torch::Tensor positions, torch::Tensor ctx_lens) {
+    const int64_t n = host_ids.numel();
+    for (auto& t : {host_ids, host_positions})
+        if (!t.is_cpu() || t.scalar_type() != torch::kInt32 || !t.is_contiguous() || t.numel() != n || n < 1) return false;
+    for (auto& t : {ids, positions, ctx_lens}) TORCH_CHECK(t.is_cuda() && t.scalar_type() == torch::kInt32 && t.is_contiguous() && t.numel() >= n, "state: CUDA int32, at least n entries");
+    c10::cuda::CUDAGuard g(ids.device());
+    SKY_CUDA_CHECK(launch_step_inputs(host_ids.data_ptr<int>(), host_positions.data_ptr<int>(), ids.data_ptr<int>(), positions.data_ptr<int>(),
+                                      ctx_lens.data_ptr<int>(), (int)n, cur_stream()));
+    return true;
+}
+
 // ---- GEMM ----
 // ss_in / ss_out: fp32 vectors of at least M entries (see GemmNormFuse); residual: y is the residual stream, updated in place.
 static void gemm(torch::Tensor x, torch::Tensor w, torch::Tensor y, int splits, bool gated, c10::optional<torch::Tensor> workspace,
@@ -566,6 +584,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     m.def("rope_append", &rope_append);
     m.def("silu_mul", &silu_mul);
     m.def("embedding", &embedding);
+    m.def("advance", &advance);
+    m.def("step_inputs", &step_inputs);
     m.def("argmax", &argmax);
     m.def("sample", &sample, py::arg("logits"), py::arg("out"), py::arg("temperature"), py::arg("seed"), py::arg("positions") = py::none());
     m.def("gemm", &gemm, py::arg("x"), py::arg("w"), py::arg("y"), py::arg("splits"), py::arg("gated"), py::arg("workspace"), py::arg("counters"),

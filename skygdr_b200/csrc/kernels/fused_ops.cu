@@ -340,4 +340,32 @@ cudaError_t launch_argmax(const __nv_bfloat16* logits, int* out, int rows, int v
     return launch_pdl_cluster(pick_kernel<false>, dim3(rows, 1, s), dim3(PICK_THREADS), 0, stream, s, logits, out, vocab, row_stride, 1.0f, 0u, (const int*)nullptr);
 }
 
+// The state of a decode batch between two steps: a few hundred bytes, so these are launches and nothing else; one each, where three
+// element-wise kernels and two copies took 1.5 us apiece with gaps as long between them.
+__global__ void __launch_bounds__(256) advance_kernel(const int* __restrict__ next_ids, int* ids, int* positions, int* ctx_lens, int n) {
+    pdl_trigger();
+    pdl_wait();
+    const int i = blockIdx.x * 256 + threadIdx.x;
+    if (i >= n) return;
+    ids[i] = next_ids[i];
+    positions[i] += 1;
+    ctx_lens[i] += 1;
+}
+cudaError_t launch_advance(const int* next_ids, int* ids, int* positions, int* ctx_lens, int n, cudaStream_t stream) {
+    if (n < 1) return cudaErrorInvalidValue;
+    return launch_pdl(advance_kernel, dim3((n + 255) / 256), dim3(256), 0, stream, next_ids, ids, positions, ctx_lens, n);
+}
+
+__global__ void __launch_bounds__(256) ctx_from_positions_kernel(const int* __restrict__ positions, int* __restrict__ ctx_lens, int n) {
+    const int i = blockIdx.x * 256 + threadIdx.x;
+    if (i < n) ctx_lens[i] = positions[i] + 1;
+}
+cudaError_t launch_step_inputs(const int* host_ids, const int* host_positions, int* ids, int* positions, int* ctx_lens, int n, cudaStream_t stream) {
+    if (n < 1) return cudaErrorInvalidValue;
+    if (cudaError_t e = cudaMemcpyAsync(ids, host_ids, (size_t)n * 4, cudaMemcpyHostToDevice, stream); e != cudaSuccess) return e;
+    if (cudaError_t e = cudaMemcpyAsync(positions, host_positions, (size_t)n * 4, cudaMemcpyHostToDevice, stream); e != cudaSuccess) return e;
+    ctx_from_positions_kernel<<<(n + 255) / 256, 256, 0, stream>>>(positions, ctx_lens, n);
+    return cudaGetLastError();
+}
+
 }  // namespace sky

@@ -61,4 +61,8 @@ cudaError_t launch_argmax(const __nv_bfloat16* logits, int* out, int rows, int v
 // of (seed, positions[r] or 0, r, column). Deterministic for given arguments; temperature > 0.
 cudaError_t launch_sample(const __nv_bfloat16* logits, int* out, int rows, int vocab, long long row_stride, float temperature,
                           unsigned int seed, const int* positions, cudaStream_t stream);
+// After a step: ids = next_ids, positions and ctx_lens advance by one.
+cudaError_t launch_advance(const int* next_ids, int* ids, int* positions, int* ctx_lens, int n, cudaStream_t stream);
+// Before a step: ids and positions from host memory, ctx_lens = positions + 1.
+cudaError_t launch_step_inputs(const int* host_ids, const int* host_positions, int* ids, int* positions, int* ctx_lens, int n, cudaStream_t stream);
 }  // namespace sky

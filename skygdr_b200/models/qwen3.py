@@ -269,6 +269,9 @@ class Qwen3Decoder:
             ops.argmax(self.logits[:b], out=self.next_ids[:b])
 
     def _advance(self, b: int) -> None:
+        if self.ids.is_cuda:
+            load().advance(self.next_ids, self.ids, self.positions, self.ctx_lens, b)
+            return
         self.ids[:b].copy_(self.next_ids[:b])
         self.positions[:b].add_(1)
         self.ctx_lens[:b].add_(1)
@@ -597,10 +600,11 @@ class DecodeSession:
 
     def step(self) -> torch.Tensor:
         e, b = self.eng, self.batch
-        e.ids[:b].copy_(self.h_ids, non_blocking=True)
-        e.positions[:b].copy_(self.h_pos, non_blocking=True)
-        e.ctx_lens[:b].copy_(e.positions[:b])
-        e.ctx_lens[:b].add_(1)
+        if not load().step_inputs(self.h_ids, self.h_pos, e.ids, e.positions, e.ctx_lens):
+            e.ids[:b].copy_(self.h_ids, non_blocking=True)
+            e.positions[:b].copy_(self.h_pos, non_blocking=True)
+            e.ctx_lens[:b].copy_(e.positions[:b])
+            e.ctx_lens[:b].add_(1)
         e.replay()
         self.h_out.copy_(e.next_ids[:b], non_blocking=True)
         torch.cuda.current_stream(e.device).synchronize()
