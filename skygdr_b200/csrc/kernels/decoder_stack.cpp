@@ -47,18 +47,26 @@ public:
         : embed_(embed), final_norm_(final_norm), inv_freq_(inv_freq), q_heads_(q_heads), kv_heads_(kv_heads), ffn_(ffn), eps_((float)eps) {
         hidden_ = (int)embed.size(1);
         qkv_cols_ = (q_heads + 2 * kv_heads) * 128;
-        auto ok = [&](const torch::Tensor& t, std::vector<int64_t> shape) {
-            TORCH_CHECK(t.is_cuda() && t.scalar_type() == torch::kBFloat16 && t.is_contiguous() && t.sizes().vec() == shape, "weights: contiguous CUDA bf16 of the fused shapes");
-        };
-        ok(embed, {embed.size(0), hidden_});
-        ok(final_norm, {hidden_});
-        TORCH_CHECK(inv_freq.scalar_type() == torch::kFloat32 && inv_freq.numel() == 64 && inv_freq.is_cuda(), "inv_freq: 64 floats");
         for (auto& l : layers) {
             TORCH_CHECK(l.size() == 8, "qkv, o, gate_up, down, ln1, ln2, q_norm, k_norm");
-            ok(l[0], {qkv_cols_, hidden_}); ok(l[1], {hidden_, q_heads * 128}); ok(l[2], {2LL * ffn, hidden_}); ok(l[3], {hidden_, ffn});
-            ok(l[4], {hidden_}); ok(l[5], {hidden_}); ok(l[6], {128}); ok(l[7], {128});
             layers_.push_back({l[0], l[1], l[2], l[3], l[4], l[5], l[6], l[7]});
         }
+    }
+
+    // Whether the weights are what the kernels take: contiguous bf16 of the fused shapes, on one GPU. Asked before every pass, since a
+    // tensor's storage and strides can be exchanged under its holder; 70 tensors take a microsecond.
+    bool fits() const {
+        if (!embed_.is_cuda() || embed_.dim() != 2) return false;
+        auto ok = [&](const torch::Tensor& t, at::IntArrayRef shape) {
+            return t.is_cuda() && t.device() == embed_.device() && t.scalar_type() == torch::kBFloat16 && t.is_contiguous() && t.sizes() == shape;
+        };
+        const int64_t h = hidden_, q = q_heads_ * 128LL, f = ffn_;
+        bool all = ok(embed_, {embed_.size(0), h}) && ok(final_norm_, {h}) && inv_freq_.is_cuda() && inv_freq_.device() == embed_.device() &&
+                   inv_freq_.scalar_type() == torch::kFloat32 && inv_freq_.is_contiguous() && inv_freq_.numel() == 64;
+        for (auto& l : layers_)
+            all = all && ok(l.qkv, {(int64_t)qkv_cols_, h}) && ok(l.o, {h, q}) && ok(l.gate_up, {2 * f, h}) && ok(l.down, {h, f}) && ok(l.ln1, {h}) &&
+                  ok(l.ln2, {h}) && ok(l.q_norm, {128}) && ok(l.k_norm, {128});
+        return all;
     }
 
     // Runs the passes and returns the normed hidden state of every prompt's last token, [sequences][hidden].
@@ -300,6 +308,7 @@ void bind_decoder_stack(py::module_& m) {
     py::class_<DecoderStack>(m, "DecoderStack")
         .def(py::init<std::vector<std::vector<torch::Tensor>>, torch::Tensor, torch::Tensor, torch::Tensor, int, int, int, double>(), py::arg("layers"),
              py::arg("embed"), py::arg("final_norm"), py::arg("inv_freq"), py::arg("q_heads"), py::arg("kv_heads"), py::arg("ffn"), py::arg("eps"))
+        .def("fits", &DecoderStack::fits)
         .def("prefill", &DecoderStack::prefill, py::call_guard<py::gil_scoped_release>(), py::arg("ids"), py::arg("starts"), py::arg("lens"), py::arg("passes"),
              py::arg("choices"), py::arg("block_table"), py::arg("pool"), py::arg("strides"), py::arg("workspace"), py::arg("counters"),
              py::arg("gemm_status"), py::arg("attn_status"))

@@ -351,11 +351,11 @@ class Qwen3Decoder:
         now = [getattr(lw, k) for lw in w.layers for k in ("qkv", "o", "gate_up", "down", "ln1", "ln2", "q_norm", "k_norm")] + [w.embed, w.final_norm]
         held = self._stack_weights
         if held is None or len(held) != len(now) or not all(map(operator.is_, held, now)):
-            fits = bool(w.layers) and all(t is not None and t.is_cuda and t.dtype == torch.bfloat16 and t.is_contiguous() for t in now)
+            fits = bool(w.layers) and all(t is not None and t.is_cuda for t in now)
             self._stack = load().DecoderStack([now[i:i + 8] for i in range(0, len(now) - 2, 8)], w.embed, w.final_norm, self.inv_freq, self.cfg.q_heads,
                                               self.cfg.kv_heads, self.cfg.ffn, self.cfg.eps) if fits else None
             self._stack_weights = now
-        return self._stack
+        return self._stack if self._stack is not None and self._stack.fits() else None
 
     def _prefill_native(self, stack, ids: torch.Tensor, seq_lens: List[int], block_table: torch.Tensor, pool: PagedKVPool, chunk: int) -> torch.Tensor:
         from ..ops.gemm import _sms, plan, workspace_for

@@ -167,6 +167,23 @@ def test_prefill_of_few_tokens_equals_the_op_by_op_prefill(lens, layout):
     assert ((kv - kv_want)[at].norm() / kv_want[at].norm()).item() < 0.015
 
 
+def test_weights_that_the_layer_stack_does_not_take_go_op_by_op():
+    """Storage exchanged under a weight tensor, of another layout: the native drivers step aside, the next layout brings them back."""
+    from skygdr_b200 import ops
+    from skygdr_b200.models import Qwen3Config, Qwen3Decoder, Qwen3Weights
+
+    cfg = Qwen3Config.tiny(layers=2, vocab=1000)
+    w = Qwen3Weights(cfg, "cuda", seed=4, std=0.05)
+    eng = Qwen3Decoder(cfg, w, ops.PagedKVPool(cfg.geometry, 4, "hnd"), max_batch=1, max_ctx=64, attn_chunk=128)
+    assert eng._layer_stack() is not None
+    gain = w.layers[1].ln1
+    plain = gain.data
+    gain.data = plain.repeat_interleave(2)[::2]
+    assert eng._layer_stack() is None
+    gain.data = plain
+    assert eng._layer_stack() is not None
+
+
 def test_tensor_parallel_shards_tile_the_full_weights():
     from skygdr_b200.models import Qwen3Config, Qwen3Weights
 
