@@ -26,6 +26,11 @@ __device__ __forceinline__ float4 rope_freqs(const float* inv_freq, int lane) {
     return make_float4(__ldg(f), __ldg(f + 1), __ldg(f + 2), __ldg(f + 3));
 }
 
+__device__ __forceinline__ void rope_unpack(uint2 v, float* f) {
+    f[0] = __uint_as_float(v.x << 16); f[1] = __uint_as_float(v.x & 0xffff0000u);
+    f[2] = __uint_as_float(v.y << 16); f[3] = __uint_as_float(v.y & 0xffff0000u);
+}
+
 // RMSNorm of U head rows at once (their shuffles overlap); x[u]: the lane's four values. Rounded to bf16 like a separate norm kernel
 // would, so results match a layer-by-layer reference.
 template <int U>

@@ -449,6 +449,40 @@ def test_rope_qknorm_append(ops):
         assert torch.equal(pool.data[blk, 0, 1, :, slot].float(), v_ref[b])
 
 
+@pytest.mark.parametrize("tokens,Hq,Hkv,normed", [(1, 1, 1, True), (5, 5, 1, True), (7, 4, 1, False), (3, 14, 2, True), (33, 16, 4, True), (2, 7, 1, False)])
+@pytest.mark.parametrize("layout", ["hnd", "nhd"])
+def test_rope_append_over_groups_of_heads(ops, tokens, Hq, Hkv, normed, layout):
+    """Eight heads share a warp: groups with q, k and v heads in them, a last group that is not full, with and without QK-norm."""
+    torch.manual_seed(tokens)
+    pool = ops.PagedKVPool(ops.KVGeometry(layers=2, kv_heads=Hkv), tokens + 1, layout)
+    pool.data.fill_(77.0)
+    pos = torch.randint(0, 16, (tokens,), device="cuda").int()
+    table = (torch.randperm(tokens, device="cuda") + 1).int().view(tokens, 1)
+    qkv = torch.randn((tokens, (Hq + 2 * Hkv) * 128), device="cuda").bfloat16()
+    w = [(torch.rand(128, device="cuda") + 0.5).bfloat16() if normed else None for _ in range(2)]
+    inv = ops.rope_inv_freq(1e6, "cuda")
+    q = ops.rope_append(qkv, w[0], w[1], pool, 1, inv, table, pos, Hq)
+    h = qkv.view(tokens, -1, 128).float()
+    ang = pos.float()[:, None, None] * inv
+    c, sn = ang.double().cos().float(), ang.double().sin().float()
+
+    def check(got, x, weight):
+        if normed:
+            x = (x * torch.rsqrt(x.pow(2).mean(-1, keepdim=True) + 1e-6) * weight.float()).bfloat16().float()
+        a, b = x[..., :64], x[..., 64:]
+        ref = torch.cat([a * c - b * sn, b * c + a * sn], -1)
+        # the normed value may round to its neighbour (2^-8 of it at most), the result is rounded once (2^-9), sine and cosine are good to 2^-20
+        bound = 2.0 ** -8 * (a.abs() + b.abs()).repeat(1, 1, 2) + 2.0 ** -9 * ref.abs() + 1e-5
+        assert bool(((got.float() - ref).abs() <= bound).all())
+
+    check(q, h[:, :Hq], w[0])
+    pages = pool.data[table[:, 0].long(), 1]                              # [tokens][k or v][..]
+    rows = torch.stack([pages[t, :, :, int(pos[t])] if layout == "hnd" else pages[t, :, int(pos[t])] for t in range(tokens)])
+    check(rows[:, 0], h[:, Hq:Hq + Hkv], w[1])
+    assert torch.equal(rows[:, 1].float(), h[:, Hq + Hkv:])
+    assert int((pool.data != 77.0).sum()) <= tokens * 2 * Hkv * 128       # nothing else is written
+
+
 def test_silu_embedding_argmax(ops):
     torch.manual_seed(6)
     gu = torch.randn((21, 2 * 1536), dtype=torch.bfloat16, device="cuda")
