@@ -17,7 +17,7 @@
 //     row; the next projection multiplies the finished product by the row's 1 / rms (it is linear in x);
 //   * QK-norm, rotary embedding and the append to the paged cache: a tile of the QKV projection is exactly one head.
 // One B200, 8 layers of Qwen3-8B's widths, host token ids in and out, against separate kernels on the general projection: one sequence
-// 1061 -> 1008 us, 16 sequences of 2k to 16k tokens 1885 -> 1810 us, 32 of 1k to 32k 3049 -> 2626 us, 100 short ones with sampling
+// 1061 -> 954 us, 16 sequences of 2k to 16k tokens 1885 -> 1807 us, 32 of 1k to 32k 3049 -> 2626 us, 100 short ones with sampling
 // 1964 -> 1869 us; prefill of 77 tokens 2174 -> 1118 us (with the passes driven from C++).
 #include <cuda.h>
 
